@@ -1,731 +1,469 @@
 // Cross-sectional kernels: one thread block per time step (row of the [T][S]
 // layout).
-//  - Rank (cpp/Kun/Rank.hpp:13-57): the row's non-NaN values are sorted by a
-//    register/shuffle/shared-memory bitonic network over order-preserving
-//    integer keys (NaNs sort last), or for long rows an 8-bit LSD radix sort;
-//    every stock then finds its equal range;
+//  - Rank (cpp/Kun/Rank.hpp:13-57): every stock's equal range in the row's
+//    sorted non-NaN values, found by counting in value-range buckets;
 //    out = T(sum) / T(cnt) / T(n) with the integer rank sum of the range.
 //  - Scale (cpp/Kun/Scale.hpp:14-46): the sum of |x| over non-NaN stocks in
 //    stock order (sequential, as the reference adds), then x / sum.
 //  - DiffWithWeightedSum (KunQuant/ops/MiscOp.py:220-240).
 #pragma once
+#include <type_traits>
+
 #include "kun_device.cuh"
 
 namespace kun {
 
+// Order-preserving integer keys: a < b of values is a < b of keys, equal values
+// (-0 and +0 too) have one key, NaN is the greatest.
 template <typename T> struct SortKey;
 template <> struct SortKey<float> {
     using K = uint32_t;
+    static constexpr K kMax = 0xffffffffu;
+    static constexpr K kNegInf = 0x007fffffu, kPosInf = 0xff800000u;
     static __device__ __forceinline__ K enc(float x) {
-        if (x != x) return 0xffffffffu;
-        uint32_t u = __float_as_uint(x);
-        return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+        const uint32_t u = __float_as_uint(kadd(x, 0.f));  // -0 + 0 is +0
+        return x == x ? u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u) : kMax;
     }
     static __device__ __forceinline__ float dec(K k) {
-        uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-        return __uint_as_float(u);
+        return __uint_as_float(k ^ ((uint32_t)((int32_t)~k >> 31) | 0x80000000u));
     }
-    static constexpr K kMax = 0xffffffffu;
+    static __device__ __forceinline__ int bits(K k) { return 32 - __clz((int)k); }
 };
 template <> struct SortKey<double> {
     using K = unsigned long long;
+    static constexpr K kMax = ~0ull;
+    static constexpr K kNegInf = 0x000fffffffffffffull, kPosInf = 0xfff0000000000000ull;
     static __device__ __forceinline__ K enc(double x) {
-        if (x != x) return ~0ull;
-        unsigned long long u = (unsigned long long)__double_as_longlong(x);
-        return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
+        const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+        if ((u & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) return kMax;
+        const K k = u ^ ((K)((long long)u >> 63) | 0x8000000000000000ull);
+        return k == 0x7fffffffffffffffull ? 0x8000000000000000ull : k;  // -0
     }
     static __device__ __forceinline__ double dec(K k) {
-        unsigned long long u = (k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k;
-        return __longlong_as_double((long long)u);
+        return __longlong_as_double((long long)(k ^ ((K)((long long)~k >> 63) | 0x8000000000000000ull)));
     }
-    static constexpr K kMax = ~0ull;
+    static __device__ __forceinline__ int bits(K k) { return 64 - __clzll((long long)k); }
 };
 
-constexpr int kRankThreads = 1024;
 // dynamic shared memory above which a launch first raises the kernel's
 // limit: 48 KB less room for the kernels' static arrays
 constexpr size_t kSmemOptIn = 40 * 1024;
-constexpr int kRadixMinP = 2048;  // rows at least this long (padded) use the radix sort
-__host__ __device__ inline int skew(int p) { return p + (p >> 5); }
-// keys per thread for a sort of P keys by kRankThreads threads
-__host__ __device__ inline int rank_items(int P) {
-    return P <= 8 * kRankThreads ? 8 : (P <= 16 * kRankThreads ? 16 : 32);
+
+// Rank of one row by one block, without sorting it.  A value's rank start is
+// the number of smaller values in its row and its end adds the equal ones:
+// exactly the equal range that the reference searches for in the sorted row
+// (cpp/Kun/Rank.hpp:40-53), so the result is the sort's bit for bit.
+//
+//  1. Every thread holds ITEMS values of the row in registers; the block finds
+//     the row's least and greatest finite value and the number of non-NaN ones.
+//  2. Each value goes to one of B = threads x ITEMS buckets by a monotone map:
+//     linear in the value, or linear in its order-preserving integer key
+//     (logarithmic in the value) for rows of one sign crowded towards zero.
+//     The first value of a bucket is its representative.
+//  3. The counters are scanned; a value that differs from its bucket's
+//     representative takes a place among such values.  Where there is none
+//     the scan alone gives the ranks, so ties cost nothing, however many.
+//  4. Those values are scattered by bucket, and every value of their buckets
+//     counts the smaller and equal ones among them.
+//
+// When a bucket holds more than kRankPoor values unlike its representative,
+// the map is refined (rank_refine), then the other map is tried and refined; a row that none of the four spreads is sorted
+// in shared memory (rank_row_sorted).  Bound by the issue rate: about 235
+// instructions a value with 75% of the issue slots taken at 8192 stocks, so the
+// block is as small as the row allows and several rows share an SM: 8 values a
+// thread up to 4096 stocks and 16 above.  Shared memory: B keys
+// (representatives, then the scattered keys over them), B counters and B
+// scanned counts, 10 bytes a value in fp32.  Normal values, against a bitonic
+// network in 1024-thread blocks up to 1024 stocks and, above, buckets with a
+// radix sort behind them in one 1024-thread block an SM: 997 stocks x 1251
+// rows 16 us (132), 3000 x 1500 41 us (88), 8192 x 2500 167 us (336), the same
+// with 10 tied values 120 us (530); fp64 801 x 1000 22 us (244).
+constexpr int kRankMaxStocks = 16384;
+constexpr int kRankPoor = 20;   // counting up to this many neighbours costs less than another map
+constexpr int kRankWorst = 96;  // counting 96 neighbours costs about as much as sorting the row
+
+__host__ __device__ inline int rank_threads(int S, int items) {
+    const int w = (S + items * 32 - 1) / (items * 32);
+    return (w < 1 ? 1 : w) * 32;
 }
-// key slots of a rank block's shared memory for rows padded to P: the radix
-// sort works on all kRankThreads * ITEMS positions
-__host__ __device__ inline int rank_key_slots(int P) {
-    return (P >= kRadixMinP ? skew(kRankThreads * rank_items(P)) : skew(P)) + 1;
+template <typename T> __host__ __device__ inline size_t rank_smem_bytes(int nt, int items) {
+    return (size_t)nt * items * (sizeof(T) + sizeof(uint32_t) + sizeof(uint16_t));
 }
 
-// Rank of one row by the whole block.  The row's keys (NaN -> max key) are
-// sorted with a bitonic network over P = a power of two >= the row length:
-// thread t holds positions [t*ITEMS, (t+1)*ITEMS) in registers, so the
-// network's exchanges at distance j < ITEMS stay in registers, j < 32*ITEMS
-// go through warp shuffles, and only the longer ones pass through shared
-// memory (keys[e*nt + t], conflict-free) with a block barrier.  Each stock
-// then binary-searches the equal range of its value in the sorted keys.
-template <typename K>
-__device__ __forceinline__ void bitonic_keep(K &mine, K other, bool lower, bool up) {
-    K mn = other < mine ? other : mine, mx = other < mine ? mine : other;
-    mine = (lower == up) ? mn : mx;
+// register budget (launch bounds): 40 a thread for 8 values in fp32, so that
+// three 512-thread blocks or their like share an SM, else 64
+template <typename T> constexpr int rank_min_blocks(int items, int maxt) {
+    return maxt == 1024 ? 1 : (items <= 8 && sizeof(T) == 4 ? 3 : 2);
 }
 
-// out[i] from the sorted non-NaN values (at(p), p < n): the average rank of
-// x's equal range over n (cpp/Kun/Rank.hpp:40-53)
-template <typename T, typename At>
-__device__ __forceinline__ void rank_from_sorted(const T *__restrict__ row, T *__restrict__ orow, long long S, int n,
-                                                 At at) {
-    for (long long i = threadIdx.x; i < S; i += blockDim.x) {
-        T x = row[i];
-        T res;
-        if (x != x) {
-            res = knan<T>();
-        } else {
-            int lo = 0, hi = n;
-            while (lo < hi) { int m = (lo + hi) >> 1; if (at(m) < x) lo = m + 1; else hi = m; }
-            long long start = lo;
-            hi = n;
-            while (lo < hi) { int m = (lo + hi) >> 1; if (x < at(m)) hi = m; else lo = m + 1; }
-            long long end = lo;
-            long long sum = (start + end + 1) * (end - start) / 2;
-            res = kdiv(kdiv((T)sum, (T)(end - start)), (T)n);
-        }
-        orow[i] = res;
+// block barriers over the first nt threads (warps past them have left)
+__device__ __forceinline__ void rank_sync(int nt) {
+    if (nt == 32) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+}
+__device__ __forceinline__ bool rank_sync_or(int nt, bool p) {
+    if (nt == 32) {
+        const bool any = __any_sync(0xffffffffu, p);
+        __syncwarp();
+        return any;
     }
-    __syncthreads();
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((int)p), "r"(nt)
+        : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ uint32_t warp_min_key(uint32_t k) { return __reduce_min_sync(0xffffffffu, k); }
+__device__ __forceinline__ uint32_t warp_max_key(uint32_t k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, k, o);
+        k = x < k ? x : k;
+    }
+    return k;
+}
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, k, o);
+        k = x > k ? x : k;
+    }
+    return k;
+}
+// T(sum) / T(cnt) / T(n) of the equal range [less, less + eq) with the integer
+// rank sum; eq = 1 leaves one division (x / 1 is x).  The sum stays below
+// 2^31: less + eq <= n <= 16384.  The division by the row's n is Markstein's
+// (IBM J. Res. Dev. 34, 1990): with r = 1/n rounded to nearest and a residual
+// by FMA, q + (s - q n) r is the correctly rounded quotient.
+template <typename T> struct RankDivisor;
+template <> struct RankDivisor<float> {
+    float n, r;
+    __device__ __forceinline__ explicit RankDivisor(int cnt) {
+        n = (float)cnt;
+        r = __frcp_rn(n);
+    }
+    __device__ __forceinline__ float operator()(float s) const {
+        const float q = __fmul_rn(s, r);
+        return __fmaf_rn(__fmaf_rn(-q, n, s), r, q);
+    }
+};
+template <> struct RankDivisor<double> {
+    double n, r;
+    __device__ __forceinline__ explicit RankDivisor(int cnt) {
+        n = (double)cnt;
+        r = __drcp_rn(n);
+    }
+    __device__ __forceinline__ double operator()(double s) const {
+        const double q = __dmul_rn(s, r);
+        return __fma_rn(__fma_rn(-q, n, s), r, q);
+    }
+};
+template <typename T> __device__ __forceinline__ T rank_value(uint32_t less, uint32_t eq, const RankDivisor<T> &n) {
+    T s = (T)(int)(less + 1);
+    if (eq != 1) s = kdiv((T)(int)((2 * less + eq + 1) * eq / 2), (T)(int)eq);
+    return n(s);
 }
 
-template <typename T, int ITEMS>
-__device__ __forceinline__ void rank_one_row(const T *__restrict__ row, T *__restrict__ orow, long long S, int P,
-                                             typename SortKey<T>::K *keys, int *cnt_warp) {
+// The row's keys sorted in shared memory (a bitonic network whose every
+// exchange puts the smaller key first, so that it needs no padding), then two
+// binary searches a value.  For rows that neither bucket map spreads.
+template <typename T, typename Out>
+__device__ __forceinline__ void rank_row_sorted(const T *__restrict__ row, int S, int n, int nt,
+                                                typename SortKey<T>::K *keys, Out out) {
     using SK = SortKey<T>;
     using K = typename SK::K;
     const int tid = threadIdx.x;
-    const int nt = P / ITEMS;  // threads holding keys (P >= ITEMS)
-    K r[ITEMS];
-    int local = 0;
-#pragma unroll
-    for (int e = 0; e < ITEMS; e++) {
-        r[e] = SK::kMax;
-        const long long i = (long long)tid * ITEMS + e;
-        if (tid < nt && i < S) {
-            T x = row[i];
-            r[e] = SK::enc(x);
-            local += (x == x);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((tid & 31) == 0) cnt_warp[tid >> 5] = local;
-    __syncthreads();
-    int n = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) n += cnt_warp[w];
+    const RankDivisor<T> over_n(n);
+    for (int i = tid; i < S; i += nt) keys[i] = SK::enc(row[i]);
+    rank_sync(nt);
+    int P = 1;
+    while (P < S) P <<= 1;
     for (int k = 2; k <= P; k <<= 1) {
-        for (int j = k >> 1; j >= ITEMS; j >>= 1) {
-            if (j >= ITEMS * 32) {
-                const int m = j / ITEMS;
-                if (tid < nt) {
-#pragma unroll
-                    for (int e = 0; e < ITEMS; e++) keys[e * nt + tid] = r[e];
-                }
-                __syncthreads();
-                if (tid < nt) {
-                    const int pt = tid ^ m;
-                    const bool lower = (tid & m) == 0;
-#pragma unroll
-                    for (int e = 0; e < ITEMS; e++) {
-                        const int i = tid * ITEMS + e;
-                        bitonic_keep(r[e], keys[e * nt + pt], lower, (i & k) == 0);
-                    }
-                }
-                __syncthreads();
-            } else {
-                const int m = j / ITEMS;
-                const bool lower = (tid & m) == 0;
-#pragma unroll
-                for (int e = 0; e < ITEMS; e++) {
-                    const int i = tid * ITEMS + e;
-                    K o = __shfl_xor_sync(0xffffffffu, r[e], m);
-                    bitonic_keep(r[e], o, lower, (i & k) == 0);
-                }
-            }
-        }
-        // distances below ITEMS: within the thread, unrolled so that r stays
-        // in registers
-#pragma unroll
-        for (int j = ITEMS / 2; j > 0; j >>= 1) {
-            if (j < k) {
-#pragma unroll
-                for (int e = 0; e < ITEMS; e++) {
-                    if ((e & j) == 0) {
-                        const int i = tid * ITEMS + e;
-                        const bool up = (i & k) == 0;
-                        K a = r[e], b = r[e ^ j];
-                        if ((a > b) == up) {
-                            r[e] = b;
-                            r[e ^ j] = a;
-                        }
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int q = tid; q < P / 2; q += nt) {
+                const int i = (q & -j) * 2 + (q & (j - 1));
+                const int o = j == (k >> 1) ? i ^ (k - 1) : i + j;  // mirrored in the first step of a merge
+                if (o < S) {
+                    const K a = keys[i], b = keys[o];
+                    if (b < a) {
+                        keys[i] = b;
+                        keys[o] = a;
                     }
                 }
             }
+            rank_sync(nt);
         }
     }
-    // sorted position p = t*ITEMS + e lives at keys[e*nt + t]
-    if (tid < nt) {
-#pragma unroll
-        for (int e = 0; e < ITEMS; e++) keys[e * nt + tid] = r[e];
+    for (int i = tid; i < S; i += nt) {
+        const K x = SK::enc(row[i]);
+        T res = knan<T>();
+        if (x != SK::kMax) {
+            int lo = 0, hi = n;
+            while (lo < hi) { const int m = (lo + hi) >> 1; if (keys[m] < x) lo = m + 1; else hi = m; }
+            const int start = lo;
+            hi = n;
+            while (lo < hi) { const int m = (lo + hi) >> 1; if (x < keys[m]) hi = m; else lo = m + 1; }
+            res = rank_value<T>((uint32_t)start, (uint32_t)(lo - start), over_n);
+        }
+        out(i, res);
     }
-    __syncthreads();
-    rank_from_sorted<T>(row, orow, S, n, [&](int p) { return SK::dec(keys[(p % ITEMS) * nt + p / ITEMS]); });
 }
 
-// Rank of one row by LSD radix sort (8-bit digits, stable), for long rows
-// where the bitonic network's P log^2 P exchanges cost more than the digit
-// passes.  blockDim.x must be kRankThreads.  Between passes the values sit in
-// layout order: warp w, item e, lane l holds position w*32*ITEMS + e*32 + l.
-// Only the non-NaN values are sorted, each with its stock index, and only
-// the digits in which they differ are passed over.  A pass counts digits per
-// warp (peers of a digit found with match.any, so an item's offset is the
-// warp's running count of its digit plus its peers in lower lanes), scans
-// the counts in (digit, warp) order and scatters.  The ranks then come from
-// the sorted run of equal values around each position (two block scans)
-// instead of binary searches.  Shared memory: keys and 16-bit stock indices
-// (skewed by one slot every 32), and kRankThreads/32 x 257 digit counters.
-constexpr int kRadixHistStride = 257;  // 256 digits + 1: warps' rows skewed by one bank
-__host__ __device__ inline int radix_hist_slots() { return (kRankThreads / 32) * kRadixHistStride; }
+// counters in 16-byte groups, swizzled so that the scan's wide reads of
+// consecutive groups meet no bank twice
+__device__ __forceinline__ int rank_swizzle(int b) { return b ^ ((b >> 3) & 0x1c); }
 
+// Splits every bucket of c values into up to c by the distance of their keys
+// from its least key, in steps of a power of two: pk's buckets become the
+// finer ones.  Exact in integers, so that values a few units in the last
+// place apart (correlations of ranks) part as well as a bucket that an
+// outlier made wide.  kmin: B keys over the representatives.
 template <typename T, int ITEMS>
-__device__ __forceinline__ void rank_one_row_radix(const T *__restrict__ row, T *__restrict__ orow, long long S,
-                                                   typename SortKey<T>::K *keys, uint32_t *hist,
-                                                   uint16_t *idx, int *cnt_warp) {
+__device__ __forceinline__ void rank_refine(const typename SortKey<T>::K (&k)[ITEMS], uint32_t (&pk)[ITEMS], int nt,
+                                            uint32_t *hist, const uint16_t *base, typename SortKey<T>::K *kmin) {
     using SK = SortKey<T>;
     using K = typename SK::K;
-    constexpr int NT = kRankThreads;
-    constexpr int NW = NT / 32;
-    static_assert(NT == 1024, "the digit-count scan gives each thread 8 of 256 x 32 counts");
-    constexpr int BITS = (int)sizeof(K) * 8;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    __shared__ int warp_tot[NW], warp_tot2[NW];
-    __shared__ K red_or[NW], red_and[NW];
-    K r[ITEMS];
-    uint16_t ix[ITEMS];
-    bool real[ITEMS];
-    int local = 0;
-    K o_or = 0, o_and = ~K(0);
-    const int wbase = warp * 32 * ITEMS + lane;  // layout position of item 0
 #pragma unroll
     for (int e = 0; e < ITEMS; e++) {
-        const int i = wbase + e * 32;
-        real[e] = false;
-        r[e] = SK::kMax;
-        ix[e] = (uint16_t)i;
-        if (i < S) {
-            T x = row[i];
-            if (x == x) {
-                real[e] = true;
-                r[e] = SK::enc(x);
-                local++;
-                o_or |= r[e];
-                o_and &= r[e];
-            } else {
-                orow[i] = knan<T>();
-            }
-        }
+        kmin[e * nt + threadIdx.x] = SK::kMax;
+        hist[e * nt + threadIdx.x] &= 0xffff;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        local += __shfl_xor_sync(0xffffffffu, local, o);
-        o_or |= __shfl_xor_sync(0xffffffffu, o_or, o);
-        o_and &= __shfl_xor_sync(0xffffffffu, o_and, o);
-    }
-    if (lane == 0) {
-        cnt_warp[warp] = local;
-        red_or[warp] = o_or;
-        red_and[warp] = o_and;
-    }
-    __syncthreads();
-    int n = 0;
-    K orv = 0, andv = ~K(0);
-    for (int w = 0; w < NW; w++) {
-        n += cnt_warp[w];
-        orv |= red_or[w];
-        andv &= red_and[w];
-    }
-    if (n == 0) {  // an all-NaN row: its outputs are written above
-        __syncthreads();
-        return;
-    }
-    // digits in which the values differ (at least one pass, which also
-    // compacts the non-NaN values to positions [0, n))
-    K todo = orv ^ andv;
-    if (todo == 0) todo = 1;
-    int last_shift = 0;
-    for (int sh = 0; sh < BITS; sh += 8)
-        if ((todo >> sh) & 255) last_shift = sh;
-    uint32_t *my_hist = hist + warp * kRadixHistStride;
-    for (int shift = 0; shift < BITS; shift += 8) {
-        if (((todo >> shift) & 255) == 0) continue;
-        for (int d = lane; d < 256; d += 32) my_hist[d] = 0;
-        __syncwarp();
-        // per-warp counts; off[e] = the item's place among its warp's items
-        // of the same digit, in layout order
-        uint16_t off[ITEMS];
-#pragma unroll
-        for (int e = 0; e < ITEMS; e++) {
-            const int d = real[e] ? (int)((r[e] >> shift) & 255) : 256;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
-            const int leader = __ffs(peers) - 1;
-            uint32_t base = 0;
-            if (lane == leader && d < 256) {
-                base = my_hist[d];
-                my_hist[d] = base + (uint32_t)__popc(peers);
-            }
-            base = __shfl_sync(0xffffffffu, base, leader);
-            off[e] = (uint16_t)(base + (uint32_t)__popc(peers & lt_mask));
-            __syncwarp();
-        }
-        __syncthreads();
-        // exclusive scan of the counts in (digit, warp) order: thread t takes
-        // the 8 entries of digit t/4, warps (t%4)*8 .. +8
-        {
-            const int d = tid >> 2, w0 = (tid & 3) * 8;
-            uint32_t c[8];
-            int sum = 0;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                c[j] = hist[(w0 + j) * kRadixHistStride + d];
-                sum += (int)c[j];
-            }
-            int incl = sum;
-            for (int o = 1; o < 32; o <<= 1) {
-                int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (lane == 31) warp_tot[warp] = incl;
-            __syncthreads();
-            if (tid < 32) {
-                int v = tid < NW ? warp_tot[tid] : 0;
-                int x = v;
-                for (int o = 1; o < 32; o <<= 1) {
-                    int y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (tid >= o) x += y;
-                }
-                if (tid < NW) warp_tot[tid] = x - v;  // exclusive
-            }
-            __syncthreads();
-            uint32_t run = (uint32_t)(warp_tot[warp] + incl - sum);
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                hist[(w0 + j) * kRadixHistStride + d] = run;
-                run += c[j];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int e = 0; e < ITEMS; e++) {
-            if (real[e]) {
-                const int d = (int)((r[e] >> shift) & 255);
-                const int pos = skew((int)my_hist[d] + off[e]);
-                keys[pos] = r[e];
-                idx[pos] = ix[e];
-            }
-        }
-        __syncthreads();
-        if (shift != last_shift) {
-#pragma unroll
-            for (int e = 0; e < ITEMS; e++) {
-                const int p = wbase + e * 32;
-                real[e] = p < n;
-                if (real[e]) {
-                    r[e] = keys[skew(p)];
-                    ix[e] = idx[skew(p)];
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // Equal runs of the sorted values: start(p) = the last run boundary at or
-    // before p (block max-scan), end(p) = one past the run (block min-scan
-    // from the right).  Equality is the values' (-0 == +0), not the keys'.
-    T v[ITEMS];
+    rank_sync(nt);
 #pragma unroll
     for (int e = 0; e < ITEMS; e++) {
-        const int p = tid * ITEMS + e;
-        v[e] = p < n ? SK::dec(keys[skew(p)]) : T(0);
+        pk[e] &= 0x3fff;
+        if (k[e] != SK::kMax) atomicMin(&kmin[pk[e]], k[e]);
     }
-    const int p0 = tid * ITEMS;
-    const T before = (p0 > 0 && p0 - 1 < n) ? SK::dec(keys[skew(p0 - 1)]) : T(0);
-    const T after = (p0 + ITEMS < n) ? SK::dec(keys[skew(p0 + ITEMS)]) : T(0);
-    int st[ITEMS], en[ITEMS];
-    int m = -1;
-#pragma unroll
-    for (int e = 0; e < ITEMS; e++) {
-        const int p = p0 + e;
-        const T prev = e == 0 ? before : v[e - 1];
-        if (p < n && (p == 0 || !(v[e] == prev))) m = p;
-        st[e] = m;
-    }
-    int mn = 1 << 30;
-#pragma unroll
-    for (int e = ITEMS - 1; e >= 0; e--) {
-        const int p = p0 + e;
-        const T next = e == ITEMS - 1 ? after : v[e + 1];
-        if (p < n && (p == n - 1 || !(v[e] == next))) mn = p + 1;
-        en[e] = mn;
-    }
-    // forward exclusive max over threads of m, backward exclusive min of mn
-    int fx = m, bx = mn;
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, fx, o);
-        if (lane >= o) fx = max(fx, y);
-        int z = __shfl_down_sync(0xffffffffu, bx, o);
-        if (lane + o < 32) bx = min(bx, z);
-    }
-    if (lane == 31) warp_tot[warp] = fx;
-    if (lane == 0) warp_tot2[warp] = bx;
-    int fex = __shfl_up_sync(0xffffffffu, fx, 1);
-    int bex = __shfl_down_sync(0xffffffffu, bx, 1);
-    if (lane == 0) fex = -1;
-    if (lane == 31) bex = 1 << 30;
-    __syncthreads();
-    if (tid < 32) {
-        int a = warp_tot[tid], b = warp_tot2[tid];
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, a, o);
-            if (tid >= o) a = max(a, y);
-            int z = __shfl_down_sync(0xffffffffu, b, o);
-            if (tid + o < 32) b = min(b, z);
-        }
-        int ae = __shfl_up_sync(0xffffffffu, a, 1);
-        int be = __shfl_down_sync(0xffffffffu, b, 1);
-        warp_tot[tid] = tid == 0 ? -1 : ae;
-        warp_tot2[tid] = tid == 31 ? (1 << 30) : be;
-    }
-    __syncthreads();
-    const int start_in = max(fex, warp_tot[warp]);
-    const int end_in = min(bex, warp_tot2[warp]);
-    T res[ITEMS];
-    int sidx[ITEMS];
-#pragma unroll
-    for (int e = 0; e < ITEMS; e++) {
-        const int p = p0 + e;
-        sidx[e] = -1;
-        if (p < n) {
-            const long long start = max(st[e], start_in);
-            const long long end = min(en[e], end_in);
-            const long long sum = (start + end + 1) * (end - start) / 2;
-            res[e] = kdiv(kdiv((T)sum, (T)(end - start)), (T)n);
-            sidx[e] = idx[skew(p)];
-        }
-    }
-    // the results go to shared memory by stock index (over the keys, no
-    // longer needed), then out in one coalesced pass over the row
-    __syncthreads();
-    T *out_s = reinterpret_cast<T *>(keys);
+    rank_sync(nt);
 #pragma unroll
     for (int e = 0; e < ITEMS; e++)
-        if (sidx[e] >= 0) out_s[sidx[e]] = res[e];
-    __syncthreads();
-    for (long long i = tid; i < S; i += NT) {
-        const T x = row[i];
-        orow[i] = x == x ? out_s[i] : knan<T>();
-    }
-    __syncthreads();
-}
-
-// Rank of one long row without sorting it: each non-NaN value goes to one
-// of kBucketN buckets by a monotone map of its value, and from the bucket
-// counts' exclusive scan a value's rank start is the number of values in
-// lower buckets plus those in its own bucket that are smaller; its end adds
-// the equal ones.  These are exactly the start and end of its equal range in
-// the sorted row (cpp/Kun/Rank.hpp:40-53), so the result is the sort's bit
-// for bit.  Two maps are counted and the one with the smaller largest bucket
-// is used: linear in the value (floor((x - min) * scale), monotone because
-// each rounded step is) for values spread evenly, and linear in the
-// order-preserving key (logarithmic in the value; -0 keyed as +0 so equal
-// values share a bucket) for values spread over many binades.  Work is O(n)
-// plus the bucket sizes; a row whose largest bucket under both maps holds
-// more than kBucketMax values (heavy ties, outliers) is left to the radix
-// sort: the function then returns false before writing anything.  Shared
-// memory: the bucketed values over `keys`, the two maps' counts and the fill
-// counters over `counters`.
-constexpr int kBucketLog = 11;
-constexpr int kBucketN = 1 << kBucketLog;
-constexpr int kBucketMax = 48;
-
-template <typename T, int ITEMS>
-__device__ __forceinline__ bool rank_one_row_bucket(const T *__restrict__ row, T *__restrict__ orow, long long S,
-                                                    typename SortKey<T>::K *keys, uint32_t *counters) {
-    using SK = SortKey<T>;
-    using K = typename SK::K;
-    constexpr int NT = kRankThreads;
-    constexpr int NW = NT / 32;
-    static_assert(kBucketN * 3 <= (NT / 32) * kRadixHistStride, "bucket counters fit the radix counters");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ K red_lo[NW], red_hi[NW];
-    __shared__ T red_vlo[NW], red_vhi[NW];
-    __shared__ int red_n[NW], red_c[NW], red_c2[NW];
-    __shared__ int scan_w[NW];
-    uint32_t *hist_v = counters, *hist_k = counters + kBucketN, *fill = counters + 2 * kBucketN;
-    T v[ITEMS];
-    K k[ITEMS];
-    int local = 0;
-    K lo = SK::kMax, hi = 0;
-    T vlo = kinf<T>(), vhi = -kinf<T>();
+        if (k[e] != SK::kMax)  // the count is below the bits
+            atomicMax(&hist[pk[e]], (hist[pk[e]] & 0xffff) | (uint32_t)SK::bits(k[e] - kmin[pk[e]]) << 16);
+    rank_sync(nt);
 #pragma unroll
     for (int e = 0; e < ITEMS; e++) {
-        const long long i = (long long)e * NT + tid;
-        v[e] = knan<T>();
-        k[e] = 0;
-        if (i < S) {
-            const T x = row[i];
-            v[e] = x;
-            if (x == x) {
-                k[e] = SK::enc(x == T(0) ? T(0) : x);
-                local++;
+        if (k[e] != SK::kMax) {
+            const uint32_t w = hist[pk[e]];
+            const int shift = (int)(w >> 16) - (31 - __clz((int)(w & 0xffff)));
+            const K d = k[e] - kmin[pk[e]];
+            pk[e] = (uint32_t)rank_swizzle(base[pk[e]] + (int)(d >> (shift > 0 ? shift : 0)));
+        }
+    }
+}
+
+// The bucket maps of a row, 1 .. B - 2 for finite values, monotone over all:
+// -inf is 0, +inf the last or beside the greatest.  In float for both types
+// (rounding to float is monotone, and FP64 arithmetic is slow here).
+template <typename T> struct RankMap {
+    using SK = SortKey<T>;
+    using K = typename SK::K;
+    bool by_key;
+    int shift;  // key distances to 32 bits
+    float scale, top;
+    K lo;
+    T vlo;
+    __device__ __forceinline__ RankMap(bool by_key_, K lo_, K hi, int B) : by_key(by_key_), lo(lo_), vlo(SK::dec(lo_)) {
+        shift = SK::bits(hi - lo) > 32 ? SK::bits(hi - lo) - 32 : 0;
+        const float range = by_key ? __uint2float_rn((uint32_t)((hi - lo) >> shift)) : (float)ksub(SK::dec(hi), vlo);
+        top = (float)(B - 2);
+        scale = fminf(__fdiv_rn((float)(B - 3), range), 3e38f);  // finite: 0 * scale is 0
+    }
+    __device__ __forceinline__ int operator()(K k) const {
+        const float d = by_key ? (k < lo ? -1.f : __uint2float_rn((uint32_t)((k - lo) >> shift)))
+                               : (float)ksub(SK::dec(k), vlo);
+        return (int)fminf(fmaxf(__fmul_rn(d, scale), -1.f), top) + 1;
+    }
+};
+
+// Ranks the S <= nt * ITEMS values of a row with the block's first nt threads
+// (a multiple of 32; the others must have left) and hands each stock's rank
+// to out(i, rank).  smem: rank_smem_bytes<T>(nt, ITEMS), 16-byte aligned.
+template <typename T, int ITEMS, typename Out>
+__device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int nt, unsigned char *smem, Out out) {
+    using SK = SortKey<T>;
+    using K = typename SK::K;
+    __shared__ K red_lo[32], red_hi[32];
+    __shared__ uint32_t red_n[32], scan_w[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const int B = nt * ITEMS;
+    K *rep = reinterpret_cast<K *>(smem), *vals = rep;
+    uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)B * sizeof(K));  // count | unlike << 16
+    uint16_t *base = reinterpret_cast<uint16_t *>(hist + B);
+    K k[ITEMS];
+#pragma unroll
+    for (int e = 0; e < ITEMS; e++) {
+        const int i = e * nt + tid;
+        k[e] = i < S ? SK::enc(row[i]) : SK::kMax;
+    }
+    const T sample = row[(unsigned)(lane * S) >> 5];  // the same 32 in every warp
+    auto clear = [&]() {
+#pragma unroll
+        for (int e = 0; e < ITEMS / 4; e++) reinterpret_cast<uint4 *>(hist)[e * nt + tid] = make_uint4(0, 0, 0, 0);
+    };
+    clear();
+    // least and greatest value and the number of them; again over the finite
+    // ones for a row that has infinities
+    K lo, hi;
+    int n;
+    bool infinite = false;
+    for (;;) {
+        lo = SK::kMax, hi = 0;
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int e = 0; e < ITEMS; e++) {
+            if (k[e] != SK::kMax) cnt++;
+            if (infinite ? k[e] > SK::kNegInf && k[e] < SK::kPosInf : k[e] != SK::kMax) {
                 lo = k[e] < lo ? k[e] : lo;
                 hi = k[e] > hi ? k[e] : hi;
-                vlo = x < vlo ? x : vlo;
-                vhi = x > vhi ? x : vhi;
             }
         }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        local += __shfl_xor_sync(0xffffffffu, local, o);
-        const K l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-        lo = l2 < lo ? l2 : lo;
-        hi = h2 > hi ? h2 : hi;
-        const T vl2 = __shfl_xor_sync(0xffffffffu, vlo, o), vh2 = __shfl_xor_sync(0xffffffffu, vhi, o);
-        vlo = vl2 < vlo ? vl2 : vlo;
-        vhi = vh2 > vhi ? vh2 : vhi;
-    }
-    if (lane == 0) {
-        red_n[warp] = local;
-        red_lo[warp] = lo;
-        red_hi[warp] = hi;
-        red_vlo[warp] = vlo;
-        red_vhi[warp] = vhi;
-    }
-    for (int b = tid; b < 3 * kBucketN; b += NT) counters[b] = 0;
-    __syncthreads();
-    // warp 0 combines the warps' partials and leaves the row's in slot 0
-    if (warp == 0) {
-        local = lane < NW ? red_n[lane] : 0;
-        lo = lane < NW ? red_lo[lane] : SK::kMax;
-        hi = lane < NW ? red_hi[lane] : K(0);
-        vlo = lane < NW ? red_vlo[lane] : kinf<T>();
-        vhi = lane < NW ? red_vhi[lane] : -kinf<T>();
-        for (int o = 16; o > 0; o >>= 1) {
-            local += __shfl_xor_sync(0xffffffffu, local, o);
-            const K l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-            lo = l2 < lo ? l2 : lo;
-            hi = h2 > hi ? h2 : hi;
-            const T vl2 = __shfl_xor_sync(0xffffffffu, vlo, o), vh2 = __shfl_xor_sync(0xffffffffu, vhi, o);
-            vlo = vl2 < vlo ? vl2 : vlo;
-            vhi = vh2 > vhi ? vh2 : vhi;
+        lo = warp_min_key(lo);
+        hi = warp_max_key(hi);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (nw > 1) {
+            if (lane == 0) {
+                red_lo[warp] = lo;
+                red_hi[warp] = hi;
+                red_n[warp] = cnt;
+            }
+            rank_sync(nt);
+            lo = warp_min_key(lane < nw ? red_lo[lane] : SK::kMax);
+            hi = warp_max_key(lane < nw ? red_hi[lane] : K(0));
+            cnt = __reduce_add_sync(0xffffffffu, lane < nw ? red_n[lane] : 0u);
+        } else {
+            __syncwarp();
         }
-        if (lane == 0) {
-            red_n[0] = local;
-            red_lo[0] = lo;
-            red_hi[0] = hi;
-            red_vlo[0] = vlo;
-            red_vhi[0] = vhi;
-        }
+        n = (int)cnt;
+        if (infinite || n == 0 || (lo > SK::kNegInf && hi < SK::kPosInf)) break;
+        infinite = true;
+        rank_sync(nt);
     }
-    __syncthreads();
-    const int n = red_n[0];
-    lo = red_lo[0];
-    hi = red_hi[0];
-    vlo = red_vlo[0];
-    vhi = red_vhi[0];
-    if (n > 0) {
-        const K range = hi - lo;
-        int bits = 0;
-        while (bits < (int)(sizeof(K) * 8) && (range >> bits) != 0) bits++;
-        const int shift = bits > kBucketLog ? bits - kBucketLog : 0;
-        // linear map: scale so that the largest value lands in the last
-        // bucket (a non-finite or zero spread puts every value in bucket 0)
-        const T spread = vhi - vlo;
-        const T scale = (spread > T(0) && spread < kinf<T>()) ? T(kBucketN - 1) / spread : T(0);
-        auto bucket_v = [&](T x) {
-            const T f = (x - vlo) * scale;
-            const int b = f >= T(kBucketN - 1) ? kBucketN - 1 : (f > T(0) ? (int)f : 0);
-            return b;
-        };
-        auto bucket_k = [&](K key) { return (int)((key - lo) >> shift); };
+    const RankDivisor<T> over_n(n);
+    if (n == 0 || (lo == hi && !infinite)) {  // no values, or one value throughout
+        const T res = n ? rank_value<T>(0u, (uint32_t)n, over_n) : knan<T>();
+#pragma unroll
+        for (int e = 0; e < ITEMS; e++) {
+            const int i = e * nt + tid;
+            if (i < S) out(i, k[e] != SK::kMax ? res : knan<T>());
+        }
+        return;
+    }
+    if (lo > hi) lo = hi = SK::enc(T(0));  // infinities alone
+    // by key: values of one sign most of which (20 of the 32 looked at) lie in
+    // the range's sixteenth nearest zero, and a spread that float does not hold
+    // (then by key only)
+    const float vlo = (float)SK::dec(lo), spread = (float)ksub(SK::dec(hi), SK::dec(lo));
+    const bool wide = !(spread < kinf<float>());
+    const float from = sample >= T(0) ? (float)sample - vlo : (float)SK::dec(hi) - (float)sample;
+    const bool key_first = wide || (((hi ^ lo) >> (sizeof(K) * 8 - 1)) == 0 &&
+                                    __popc(__ballot_sync(0xffffffffu, from < spread * 0.0625f)) >= 20);
+    uint32_t pk[ITEMS];  // bucket | place << 14 | relation to the representative << 30 (1 below, 2 above)
+    bool sorted = false;
+    for (int attempt = 0;; attempt++) {
+        if (attempt & 1) {
+            rank_refine<T, ITEMS>(k, pk, nt, hist, base, rep);
+        } else {
+            const RankMap<T> map(wide || key_first != (attempt == 2), lo, hi, B);
+#pragma unroll
+            for (int e = 0; e < ITEMS; e++) pk[e] = (uint32_t)rank_swizzle(map(k[e]));
+        }
+        if (attempt) {
+            rank_sync(nt);
+            clear();
+            rank_sync(nt);
+        }
 #pragma unroll
         for (int e = 0; e < ITEMS; e++)
-            if (v[e] == v[e]) {
-                atomicAdd(&hist_v[bucket_v(v[e])], 1u);
-                atomicAdd(&hist_k[bucket_k(k[e])], 1u);
-            }
-        __syncthreads();
-        // the map with the smaller largest bucket; the radix sort if both
-        // overflow
-        int mv = 0, mk = 0;
-        for (int b = tid; b < kBucketN; b += NT) {
-            mv = max(mv, (int)hist_v[b]);
-            mk = max(mk, (int)hist_k[b]);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-            mk = max(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-        }
-        if (lane == 0) {
-            red_c[warp] = mv;
-            red_c2[warp] = mk;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            mv = lane < NW ? red_c[lane] : 0;
-            mk = lane < NW ? red_c2[lane] : 0;
-            for (int o = 16; o > 0; o >>= 1) {
-                mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-                mk = max(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-            }
-            if (lane == 0) {
-                red_c[0] = mv;
-                red_c2[0] = mk;
-            }
-        }
-        __syncthreads();
-        mv = red_c[0];
-        mk = red_c2[0];
-        if (mv > kBucketMax && mk > kBucketMax) {
-            __syncthreads();
-            return false;
-        }
-        const bool lin = mv <= mk;
-        uint32_t *hist = lin ? hist_v : hist_k;
-        // exclusive scan of the counts (kBucketN / NT per thread, in order)
-        constexpr int PER = kBucketN / NT;
-        uint32_t c[PER], sum = 0;
+            if (k[e] != SK::kMax && atomicAdd(&hist[pk[e]], 1u) == 0) rep[pk[e]] = k[e];
+        rank_sync(nt);
+        uint32_t deep = 0;
 #pragma unroll
-        for (int j = 0; j < PER; j++) {
-            c[j] = hist[tid * PER + j];
-            sum += c[j];
+        for (int e = 0; e < ITEMS; e++) {
+            const K r = rep[pk[e]];
+            if (k[e] != SK::kMax && r != k[e]) {
+                const uint32_t place = atomicAdd(&hist[pk[e]], 0x10000u) >> 16;
+                deep = max(deep, place);
+                pk[e] |= place << 14 | (k[e] < r ? 1u << 30 : 2u << 30);
+            }
+        }
+        // exclusive scan of the counts, ITEMS consecutive ones a thread
+        uint32_t sum = 0;
+#pragma unroll
+        for (int g = 0; g < ITEMS / 4; g++) {
+            const int at = tid * (ITEMS / 4) + g;
+            const uint4 q = reinterpret_cast<const uint4 *>(hist)[at ^ ((at >> 3) & 7)];
+            sum += (q.x & 0xffff) + (q.y & 0xffff) + (q.z & 0xffff) + (q.w & 0xffff);
         }
         uint32_t incl = sum;
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
-        if (lane == 31) scan_w[warp] = (int)incl;
-        __syncthreads();
-        if (tid < 32) {
-            int x = tid < NW ? scan_w[tid] : 0;
-            const int v0 = x;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (tid >= o) x += y;
-            }
-            if (tid < NW) scan_w[tid] = x - v0;
-        }
-        __syncthreads();
-        uint32_t run = (uint32_t)scan_w[warp] + incl - sum;
+        if (lane == 31) scan_w[warp] = incl;
+        rank_sync(nt);
+        uint32_t run = __reduce_add_sync(0xffffffffu, lane < warp ? scan_w[lane] : 0u) + incl - sum;
 #pragma unroll
-        for (int j = 0; j < PER; j++) {
-            hist[tid * PER + j] = run;
-            run += c[j];
+        for (int g = 0; g < ITEMS / 4; g++) {
+            const int at = tid * (ITEMS / 4) + g, sw = at ^ ((at >> 3) & 7);
+            const uint4 q = reinterpret_cast<const uint4 *>(hist)[sw];
+            const uint32_t b0 = run, b1 = b0 + (q.x & 0xffff), b2 = b1 + (q.y & 0xffff), b3 = b2 + (q.z & 0xffff);
+            run = b3 + (q.w & 0xffff);
+            reinterpret_cast<uint2 *>(base)[sw] = make_uint2(b0 | b1 << 16, b2 | b3 << 16);
         }
-        __syncthreads();
-        // the values by bucket (unordered inside a bucket)
-        T *vals = reinterpret_cast<T *>(keys);
-        int bk[ITEMS];
-#pragma unroll
-        for (int e = 0; e < ITEMS; e++) {
-            bk[e] = 0;
-            if (v[e] == v[e]) {
-                bk[e] = lin ? bucket_v(v[e]) : bucket_k(k[e]);
-                vals[hist[bk[e]] + atomicAdd(&fill[bk[e]], 1u)] = v[e];
-            }
+        if (!rank_sync_or(nt, deep >= (uint32_t)(attempt < 3 ? kRankPoor : kRankWorst))) break;
+        if (attempt == 3) {
+            sorted = true;
+            break;
         }
-        __syncthreads();
+        // a bucket that most of the row is in asks for the other map at once
+        if (attempt == 0 && rank_sync_or(nt, deep >= (uint32_t)n / 4 * 3)) attempt = 1;
+    }
+    if (sorted) {
+        rank_row_sorted<T>(row, S, n, nt, reinterpret_cast<K *>(smem), out);
+        return;
+    }
+    // the representatives are no longer needed: the values unlike them take
+    // their place
 #pragma unroll
-        for (int e = 0; e < ITEMS; e++) {
-            const long long i = (long long)e * NT + tid;
-            if (i >= S) continue;
-            T res = knan<T>();
-            if (v[e] == v[e]) {
-                const int b = bk[e];
-                const int p0 = (int)hist[b], p1 = b + 1 < kBucketN ? (int)hist[b + 1] : n;
-                int less = p0, eq = 0;
-                for (int p = p0; p < p1; p++) {
-                    const T y = vals[p];
-                    less += (y < v[e]);
-                    eq += (y == v[e]);
+    for (int e = 0; e < ITEMS; e++)
+        if (pk[e] >> 30) vals[base[pk[e] & 0x3fff] + ((pk[e] >> 14) & 0x3fff)] = k[e];
+    rank_sync(nt);
+#pragma unroll
+    for (int e = 0; e < ITEMS; e++) {
+        const int i = e * nt + tid;
+        if (i < S) {
+            const int at = pk[e] & 0x3fff;
+            const uint32_t w = hist[at], unlike = w >> 16, like = (w & 0xffff) - unlike;
+            uint32_t less = base[at], eq = like;
+            if (unlike) {
+                uint32_t same = 0;
+#pragma unroll 1
+                for (uint32_t p = less, p1 = less + unlike; p < p1; p++) {
+                    const K y = vals[p];
+                    less += (y < k[e]);
+                    same += (y == k[e]);
                 }
-                const long long start = less, end = (long long)less + eq;
-                const long long rsum = (start + end + 1) * (end - start) / 2;
-                res = kdiv(kdiv((T)rsum, (T)(end - start)), (T)n);
+                if (pk[e] >> 30) eq = same;
+                if (pk[e] >> 31) less += like;
             }
-            orow[i] = res;
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < ITEMS; e++) {
-            const long long i = (long long)e * NT + tid;
-            if (i < S) orow[i] = knan<T>();
-        }
-    }
-    __syncthreads();
-    return true;
-}
-
-// shared memory of a rank block sorting up to P keys
-template <typename T>
-inline size_t rank_smem_bytes(int P) {
-    using K = typename SortKey<T>::K;
-    size_t keys = ((size_t)rank_key_slots(P) * sizeof(K) + 15) / 16 * 16;
-    return P >= kRadixMinP ? keys + (size_t)radix_hist_slots() * sizeof(uint32_t) +
-                                 (size_t)rank_key_slots(P) * sizeof(uint16_t)
-                           : keys;
-}
-
-template <typename T, int ITEMS>
-__global__ void __launch_bounds__(kRankThreads) rank_rows(const T *__restrict__ in, T *__restrict__ out,
-                                                          long long S, long long length, int P) {
-    using K = typename SortKey<T>::K;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int cnt_warp[kRankThreads / 32];
-    K *keys = reinterpret_cast<K *>(smem_raw);
-    uint32_t *counters = reinterpret_cast<uint32_t *>(smem_raw + ((size_t)rank_key_slots(P) * sizeof(K) + 15) / 16 * 16);
-    uint16_t *idx = reinterpret_cast<uint16_t *>(counters + radix_hist_slots());
-    for (long long t = blockIdx.x; t < length; t += gridDim.x) {
-        if (P >= kRadixMinP) {
-            if (!rank_one_row_bucket<T, ITEMS>(in + t * S, out + t * S, S, keys, counters))
-                rank_one_row_radix<T, ITEMS>(in + t * S, out + t * S, S, keys, counters, idx, cnt_warp);
-        } else {
-            rank_one_row<T, ITEMS>(in + t * S, out + t * S, S, P, keys, cnt_warp);
+            out(i, k[e] != SK::kMax ? rank_value<T>(less, eq, over_n) : knan<T>());
         }
     }
 }
 
-// stream mode: one block per segment, each at its own ring row
-template <typename T, int ITEMS>
-__global__ void __launch_bounds__(kRankThreads) rank_segments(const T *__restrict__ in, int w_in, T *__restrict__ out,
-                                                              int w_out, long long cap, const int32_t *seg_off,
-                                                              const int32_t *seg_stock0, const long long *seg_tick,
-                                                              int P, const int32_t *cnt) {
-    using K = typename SortKey<T>::K;
+template <typename T> struct RankStore {
+    T *__restrict__ o;
+    __device__ __forceinline__ void operator()(int i, T r) const { o[i] = r; }
+};
+
+// rows of one [length][S] plane, a block each; blockDim.x = rank_threads(S, ITEMS)
+template <typename T, int ITEMS, int MAXT>
+__global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_rows(const T *__restrict__ in, T *__restrict__ out, int S) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int cnt_warp[kRankThreads / 32];
-    const int k = blockIdx.x;
-    if (cnt && k >= cnt[0]) return;
-    const long long len = seg_off[k + 1] - seg_off[k], s0 = seg_stock0[k], n = seg_tick[k];
-    // sort only the power of two this segment needs (P bounds every segment)
-    if (len > P) return;
-    int Pk = ITEMS;
-    while (Pk < len) Pk <<= 1;
-    K *keys = reinterpret_cast<K *>(smem_raw);
-    uint32_t *counters = reinterpret_cast<uint32_t *>(smem_raw + ((size_t)rank_key_slots(P) * sizeof(K) + 15) / 16 * 16);
-    uint16_t *idx = reinterpret_cast<uint16_t *>(counters + radix_hist_slots());
-    if (Pk >= kRadixMinP) {
-        if (!rank_one_row_bucket<T, ITEMS>(in + (n % w_in) * cap + s0, out + (n % w_out) * cap + s0, len, keys,
-                                           counters))
-            rank_one_row_radix<T, ITEMS>(in + (n % w_in) * cap + s0, out + (n % w_out) * cap + s0, len, keys,
-                                         counters, idx, cnt_warp);
-    } else
-        rank_one_row<T, ITEMS>(in + (n % w_in) * cap + s0, out + (n % w_out) * cap + s0, len, Pk, keys, cnt_warp);
+    const long long t = blockIdx.x;
+    rank_row<T, ITEMS>(in + t * S, S, (int)blockDim.x, smem_raw, RankStore<T>{out + t * S});
 }
 
 // Stream mode, several Rank stages at once: block (k, j) ranks segment k
@@ -738,39 +476,37 @@ struct RankJob {
     int32_t w_in, w_out;
 };
 
-// Segments of at most kRankSmallMax stocks go to blocks of kRankSmallThreads
-// threads (a bitonic sort of at most 1024 keys, 8 per thread); longer ones to
-// kRankThreads-thread blocks.  A step's table lists its small segments first
-// and holds their number in cnt[3].
-constexpr int kRankSmallMax = 1024;
-constexpr int kRankSmallThreads = kRankSmallMax / 8;
+template <typename T, int ITEMS, int MAXT>
+__device__ __forceinline__ void rank_segment(const T *in, int w_in, T *out, int w_out, long long cap, long long len,
+                                             long long s0, long long n, unsigned char *smem) {
+    if (len <= 0 || len > (long long)blockDim.x * ITEMS) return;
+    const int nt = rank_threads((int)len, ITEMS);
+    if ((int)threadIdx.x >= nt) return;
+    rank_row<T, ITEMS>(in + (n % w_in) * cap + s0, (int)len, nt, smem, RankStore<T>{out + (n % w_out) * cap + s0});
+}
 
-template <typename T, int ITEMS, bool SMALL>
-__global__ void __launch_bounds__(SMALL ? kRankSmallThreads : kRankThreads)
-    rank_multi_segments(const RankJob *__restrict__ jobs, long long cap, const int32_t *seg_off,
-                        const int32_t *seg_stock0, const long long *seg_tick, int P, const int32_t *cnt) {
-    using K = typename SortKey<T>::K;
+// one stage, one block per segment, each at its own ring row
+template <typename T, int ITEMS, int MAXT>
+__global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_segments(const T *in, int w_in, T *out, int w_out, long long cap,
+                                                      const int32_t *seg_off, const int32_t *seg_stock0,
+                                                      const long long *seg_tick, const int32_t *cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int cnt_warp[kRankThreads / 32];
     const int k = blockIdx.x;
-    if (cnt && (k >= cnt[0] || (SMALL ? k >= cnt[3] : k < cnt[3]))) return;
+    if (cnt && k >= cnt[0]) return;
+    rank_segment<T, ITEMS, MAXT>(in, w_in, out, w_out, cap, seg_off[k + 1] - seg_off[k], seg_stock0[k], seg_tick[k],
+                                 smem_raw);
+}
+
+template <typename T, int ITEMS, int MAXT>
+__global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_multi_segments(const RankJob *__restrict__ jobs, long long cap,
+                                                            const int32_t *seg_off, const int32_t *seg_stock0,
+                                                            const long long *seg_tick, const int32_t *cnt) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int k = blockIdx.x;
+    if (cnt && k >= cnt[0]) return;
     const RankJob jb = jobs[blockIdx.y];
-    const long long len = seg_off[k + 1] - seg_off[k], s0 = seg_stock0[k], n = seg_tick[k];
-    if (len > P || len <= 0 || (SMALL && len > kRankSmallMax)) return;
-    int Pk = ITEMS;
-    while (Pk < len) Pk <<= 1;
-    const T *in = (const T *)jb.in + (n % jb.w_in) * cap + s0;
-    T *out = (T *)jb.out + (n % jb.w_out) * cap + s0;
-    K *keys = reinterpret_cast<K *>(smem_raw);
-    uint32_t *counters = reinterpret_cast<uint32_t *>(smem_raw + ((size_t)rank_key_slots(P) * sizeof(K) + 15) / 16 * 16);
-    uint16_t *idx = reinterpret_cast<uint16_t *>(counters + radix_hist_slots());
-    if (SMALL)
-        rank_one_row<T, ITEMS>(in, out, len, Pk, keys, cnt_warp);
-    else if (Pk >= kRadixMinP) {
-        if (!rank_one_row_bucket<T, ITEMS>(in, out, len, keys, counters))
-            rank_one_row_radix<T, ITEMS>(in, out, len, keys, counters, idx, cnt_warp);
-    } else
-        rank_one_row<T, ITEMS>(in, out, len, Pk, keys, cnt_warp);
+    rank_segment<T, ITEMS, MAXT>((const T *)jb.in, jb.w_in, (T *)jb.out, jb.w_out, cap, seg_off[k + 1] - seg_off[k],
+                                 seg_stock0[k], seg_tick[k], smem_raw);
 }
 
 template <typename T>
@@ -916,17 +652,44 @@ inline int kun_num_sms() {
     return n;
 }
 
-template <typename T, int ITEMS>
-inline int launch_rank_items(const T *in, T *out, long long S, long long length, int P, cudaStream_t st) {
-    size_t smem = rank_smem_bytes<T>(P);
-    if (smem > kSmemOptIn) {
-        cudaError_t e =
-            cudaFuncSetAttribute(rank_rows<T, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
+template <typename Kernel> inline int rank_smem_limit(Kernel kernel, size_t smem) {
+    if (smem <= kSmemOptIn) return 0;
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+// The block for rows of up to S stocks: go(items, max threads).  Batch rows
+// are many, so they take few threads with many values each (throughput: the
+// phases' fixed cost is a thread's); a stream's levels wait for one row, so
+// they take 1024 threads before they take more values a thread (a level of one
+// 4096-stock segment: 9 us, 22 us before).
+template <bool LATENCY, typename Go> inline int rank_dispatch(long long S, Go go) {
+    if (S > kRankMaxStocks) return (int)cudaErrorInvalidValue;
+    using I4 = std::integral_constant<int, 4>;
+    using I8 = std::integral_constant<int, 8>;
+    using I16 = std::integral_constant<int, 16>;
+    using T512 = std::integral_constant<int, 512>;
+    using T1024 = std::integral_constant<int, 1024>;
+    if constexpr (LATENCY) {
+        if (S <= 4096) return go(I4(), T1024());
+        if (S <= 8192) return go(I8(), T1024());
+    } else {
+        if (S <= 128) return go(I4(), T512());
+        if (S <= 4096) return go(I8(), T512());
+        if (S <= 8192) return go(I16(), T512());
     }
-    long long grid = length < (long long)kun_num_sms() * 2 ? length : (long long)kun_num_sms() * 2;
-    rank_rows<T, ITEMS><<<(unsigned)grid, kRankThreads, smem, st>>>(in, out, S, length, P);
-    return (int)cudaGetLastError();
+    return go(I16(), T1024());
+}
+
+template <typename T>
+inline int launch_rank(const T *in, T *out, long long S, long long length, cudaStream_t st) {
+    return rank_dispatch<false>(S, [&](auto items, auto maxt) {
+        constexpr int I = decltype(items)::value, M = decltype(maxt)::value;
+        const int nt = rank_threads((int)S, I);
+        const size_t smem = rank_smem_bytes<T>(nt, I);
+        if (int e = rank_smem_limit(rank_rows<T, I, M>, smem)) return e;
+        rank_rows<T, I, M><<<(unsigned)length, nt, smem, st>>>(in, out, (int)S);
+        return (int)cudaGetLastError();
+    });
 }
 
 // Batch runs of several universes: the rows of one Rank stage of every job
@@ -938,74 +701,41 @@ struct RankRowsJob {
     long long S, length, row0;
 };
 
-template <typename T, int ITEMS>
-__global__ void __launch_bounds__(kRankThreads) rank_rows_multi(const RankRowsJob *__restrict__ jobs, int njobs,
-                                                                long long total_rows, int P) {
-    using K = typename SortKey<T>::K;
+// A block has the threads of the longest row; a shorter row's surplus warps
+// leave at once and its barriers count only the others.
+template <typename T, int ITEMS, int MAXT>
+__global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_rows_multi(const RankRowsJob *__restrict__ jobs, int njobs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int cnt_warp[kRankThreads / 32];
-    K *keys = reinterpret_cast<K *>(smem_raw);
-    uint32_t *counters = reinterpret_cast<uint32_t *>(smem_raw + ((size_t)rank_key_slots(P) * sizeof(K) + 15) / 16 * 16);
-    uint16_t *idx = reinterpret_cast<uint16_t *>(counters + radix_hist_slots());
-    for (long long r = blockIdx.x; r < total_rows; r += gridDim.x) {
-        int lo = 0, hi = njobs - 1;  // the job whose rows hold r
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (jobs[mid].row0 <= r) lo = mid;
-            else hi = mid - 1;
-        }
-        const RankRowsJob jb = jobs[lo];
-        const long long t = r - jb.row0, S = jb.S;
-        if (t < 0 || t >= jb.length || S <= 0 || S > P) continue;
-        const T *in = (const T *)jb.in + t * S;
-        T *out = (T *)jb.out + t * S;
-        int Pk = ITEMS;
-        while (Pk < S) Pk <<= 1;
-        if (Pk >= kRadixMinP) {
-            if (!rank_one_row_bucket<T, ITEMS>(in, out, S, keys, counters))
-                rank_one_row_radix<T, ITEMS>(in, out, S, keys, counters, idx, cnt_warp);
-        } else {
-            rank_one_row<T, ITEMS>(in, out, S, Pk, keys, cnt_warp);
-        }
+    const long long r = blockIdx.x;
+    int lo = 0, hi = njobs - 1;  // the job whose rows hold r
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].row0 <= r) lo = mid;
+        else hi = mid - 1;
     }
+    const RankRowsJob jb = jobs[lo];
+    const long long t = r - jb.row0, S = jb.S;
+    if (t < 0 || t >= jb.length || S <= 0 || S > (long long)blockDim.x * ITEMS) return;
+    const int nt = rank_threads((int)S, ITEMS);
+    if ((int)threadIdx.x >= nt) return;
+    rank_row<T, ITEMS>((const T *)jb.in + t * S, (int)S, nt, smem_raw, RankStore<T>{(T *)jb.out + t * S});
 }
 
-// max_S: the longest row of the jobs (sizes the keys per thread and the
-// shared memory)
+// max_S: the longest row of the jobs (sizes the blocks and their shared
+// memory)
 template <typename T>
 inline int launch_rank_rows_multi(const RankRowsJob *d_jobs, int njobs, long long total_rows, long long max_S,
                                   cudaStream_t st) {
     if (njobs <= 0 || total_rows <= 0) return 0;
-    int P = 8;
-    while (P < max_S) P <<= 1;
-    const size_t smem = rank_smem_bytes<T>(P);
-    if (smem > 227 * 1024 || P > 32 * kRankThreads) return (int)cudaErrorInvalidValue;
-    const long long grid = total_rows < (long long)kun_num_sms() * 2 ? total_rows : (long long)kun_num_sms() * 2;
-    auto go = [&](auto kernel) {
-        if (smem > kSmemOptIn) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-        }
-        kernel<<<(unsigned)grid, kRankThreads, smem, st>>>(d_jobs, njobs, total_rows, P);
+    if (total_rows > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+    return rank_dispatch<false>(max_S, [&](auto items, auto maxt) {
+        constexpr int I = decltype(items)::value, M = decltype(maxt)::value;
+        const int nt = rank_threads((int)max_S, I);
+        const size_t smem = rank_smem_bytes<T>(nt, I);
+        if (int e = rank_smem_limit(rank_rows_multi<T, I, M>, smem)) return e;
+        rank_rows_multi<T, I, M><<<(unsigned)total_rows, nt, smem, st>>>(d_jobs, njobs);
         return (int)cudaGetLastError();
-    };
-    switch (rank_items(P)) {
-    case 8: return go(rank_rows_multi<T, 8>);
-    case 16: return go(rank_rows_multi<T, 16>);
-    default: return go(rank_rows_multi<T, 32>);
-    }
-}
-
-template <typename T>
-inline int launch_rank(const T *in, T *out, long long S, long long length, cudaStream_t st) {
-    int P = 8;
-    while (P < S) P <<= 1;
-    if (rank_smem_bytes<T>(P) > 227 * 1024 || P > 32 * kRankThreads) return (int)cudaErrorInvalidValue;
-    switch (rank_items(P)) {
-    case 8: return launch_rank_items<T, 8>(in, out, S, length, P, st);
-    case 16: return launch_rank_items<T, 16>(in, out, S, length, P, st);
-    default: return launch_rank_items<T, 32>(in, out, S, length, P, st);
-    }
+    });
 }
 
 template <typename T>
@@ -1032,63 +762,34 @@ template <typename T>
 inline int launch_rank_segments(const T *in, int w_in, T *out, int w_out, long long cap, const int32_t *seg_off,
                                 const int32_t *seg_stock0, const long long *seg_tick, int nseg, int max_len,
                                 const int32_t *cnt, cudaStream_t st) {
-    int P = 8;
-    while (P < max_len) P <<= 1;
-    size_t smem = rank_smem_bytes<T>(P);
-    if (smem > 227 * 1024 || P > 32 * kRankThreads) return (int)cudaErrorInvalidValue;
-    auto go = [&](auto kernel) {
-        if (smem > kSmemOptIn) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-        }
-        kernel<<<(unsigned)nseg, kRankThreads, smem, st>>>(in, w_in, out, w_out, cap, seg_off, seg_stock0, seg_tick,
-                                                           P, cnt);
+    return rank_dispatch<true>(max_len, [&](auto items, auto maxt) {
+        constexpr int I = decltype(items)::value, M = decltype(maxt)::value;
+        const int nt = rank_threads(max_len, I);
+        const size_t smem = rank_smem_bytes<T>(nt, I);
+        if (int e = rank_smem_limit(rank_segments<T, I, M>, smem)) return e;
+        rank_segments<T, I, M><<<(unsigned)nseg, nt, smem, st>>>(in, w_in, out, w_out, cap, seg_off, seg_stock0,
+                                                                seg_tick, cnt);
         return (int)cudaGetLastError();
-    };
-    switch (rank_items(P)) {
-    case 8: return go(rank_segments<T, 8>);
-    case 16: return go(rank_segments<T, 16>);
-    default: return go(rank_segments<T, 32>);
-    }
+    });
 }
 
-// njobs Rank stages over the step's segments: one launch for the segments
-// of at most kRankSmallMax stocks and one for the longer ones.  With a
-// device table (cnt: nseg, stocks, longest, number of small segments) both
-// launch and each takes its part; without one every segment goes to the
-// launch that max_len picks.
+// njobs Rank stages over the step's segments in one launch (cnt: the step's
+// device table, or null when the step has exactly nseg segments)
 template <typename T>
 inline int launch_rank_multi_segments(const RankJob *d_jobs, int njobs, long long cap, const int32_t *seg_off,
                                       const int32_t *seg_stock0, const long long *seg_tick, int nseg, int max_len,
-                                      const int32_t *cnt, cudaStream_t st, cudaStream_t st_long = nullptr) {
+                                      const int32_t *cnt, cudaStream_t st) {
     if (njobs <= 0 || nseg <= 0) return 0;
     if (njobs > 65535) return (int)cudaErrorInvalidValue;
-    const dim3 grid((unsigned)nseg, (unsigned)njobs);
-    if (cnt || max_len <= kRankSmallMax) {
-        const size_t smem = rank_smem_bytes<T>(kRankSmallMax);
-        rank_multi_segments<T, 8, true><<<grid, kRankSmallThreads, smem, st>>>(d_jobs, cap, seg_off, seg_stock0,
-                                                                            seg_tick, kRankSmallMax, cnt);
-        if (cudaError_t e = cudaGetLastError()) return (int)e;
-    }
-    if (!cnt && max_len <= kRankSmallMax) return 0;
-    if (st_long) st = st_long;
-    int P = 8;
-    while (P < max_len) P <<= 1;
-    size_t smem = rank_smem_bytes<T>(P);
-    if (smem > 227 * 1024 || P > 32 * kRankThreads) return (int)cudaErrorInvalidValue;
-    auto go = [&](auto kernel) {
-        if (smem > kSmemOptIn) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-        }
-        kernel<<<grid, kRankThreads, smem, st>>>(d_jobs, cap, seg_off, seg_stock0, seg_tick, P, cnt);
+    return rank_dispatch<true>(max_len, [&](auto items, auto maxt) {
+        constexpr int I = decltype(items)::value, M = decltype(maxt)::value;
+        const int nt = rank_threads(max_len, I);
+        const size_t smem = rank_smem_bytes<T>(nt, I);
+        if (int e = rank_smem_limit(rank_multi_segments<T, I, M>, smem)) return e;
+        rank_multi_segments<T, I, M><<<dim3((unsigned)nseg, (unsigned)njobs), nt, smem, st>>>(
+            d_jobs, cap, seg_off, seg_stock0, seg_tick, cnt);
         return (int)cudaGetLastError();
-    };
-    switch (rank_items(P)) {
-    case 8: return go(rank_multi_segments<T, 8, false>);
-    case 16: return go(rank_multi_segments<T, 16, false>);
-    default: return go(rank_multi_segments<T, 32, false>);
-    }
+    });
 }
 
 template <typename T>
