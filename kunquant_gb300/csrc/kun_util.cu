@@ -4,11 +4,13 @@
 // Reference: cpp/Kun/CorrWith.hpp:12-121, cpp/Kun/Aggregration.cpp:12-106,
 // bound in Python at cpp/Python/PyBinding.cpp:396-506.
 //
-// corrWith: one block per (time row, input); the five moments are summed per
-// thread over a strided share of the stocks in two-float compensated fp32,
-// then tree-reduced.  The reference adds in stock order in plain fp32, so the
-// results agree to rounding (its own tests hold 1e-4 relative to pandas).
-// RankCorrWith first ranks each input row exactly as Rank does.
+// corrWith: one block per (time row, input); the moments are summed per thread
+// over a strided share of the stocks in two-float compensated fp32, then
+// tree-reduced.  The label row's own moments do not depend on the input: one
+// pass sums them for all.  The reference adds in stock order in plain fp32, so
+// the results agree to rounding (its own tests hold 1e-4 relative to pandas).
+// RankCorrWith ranks a row exactly as Rank does and sums the ranks from the
+// registers they are found in.
 //
 // aggregrate: one thread per (stock, group, input) walks the group's rows in
 // order, with the reference's reductions (Kahan sum, NaN-sticky min/max), so
@@ -24,7 +26,7 @@
 
 namespace kungpu {
 
-constexpr int kCorrThreads = 256;
+constexpr int kCorrThreads = 128;
 
 // element (t, s) of a [T][S] (layout 1) or [S/L][T][L] (layout 0) buffer
 __device__ __forceinline__ long long util_index(int layout, long long s, long long t, long long S, long long T,
@@ -32,54 +34,124 @@ __device__ __forceinline__ long long util_index(int layout, long long s, long lo
     return layout == 1 ? t * S + s : (s / L) * T * L + t * L + s % L;
 }
 
-__device__ __forceinline__ kun::DFloat warp_sum_df(kun::DFloat v) {
-    for (int o = 16; o > 0; o >>= 1) {
-        kun::DFloat w(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
-        v = kun::kadd(v, w);
-    }
-    return v;
-}
-
-// in[k] rows, y row source; out[k][t]
-__global__ void __launch_bounds__(kCorrThreads) corr_rows(const float *const *in, const float *y, float *const *out,
-                                                          long long S, long long T, int layout, int L) {
-    const long long t = blockIdx.x;
-    const int k = blockIdx.y;
-    const float *x = in[k];
-    kun::DFloat X, Y, X2, Y2, XY;
-    for (long long s = threadIdx.x; s < S; s += blockDim.x) {
-        const long long ix = util_index(layout, s, t, S, T, L);
-        const float a = x[ix], b = y[ix];
-        X = kun::df_add_f(X, a);
-        Y = kun::df_add_f(Y, b);
-        X2 = kun::df_add_prod(X2, a, a);
-        Y2 = kun::df_add_prod(Y2, b, b);
-        XY = kun::df_add_prod(XY, a, b);
-    }
-    __shared__ float sh[5][2][kCorrThreads / 32];
-    kun::DFloat v[5] = {X, Y, X2, Y2, XY};
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// Sums of a thread, all kept as unnormalised pairs (kun::df_acc).  A sum that
+// has left the finite range is its high part alone: the pair's error term is
+// then NaN.
+template <int N> struct CorrSums {
+    kun::DFloat v[N];
+    // one more value of every thread's sums over the block's first nt threads;
+    // thread 0 has the totals
+    __device__ __forceinline__ void reduce(int nt) {
+        __shared__ float sh[N][2][32];
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = nt >> 5;
 #pragma unroll
-    for (int q = 0; q < 5; q++) {
-        v[q] = warp_sum_df(v[q]);
-        if (lane == 0) {
-            sh[q][0][w] = v[q].hi;
-            sh[q][1][w] = v[q].lo;
+        for (int q = 0; q < N; q++) {
+            if (!isfinite(v[q].hi)) v[q].lo = 0.f;
+            v[q] = warp_sum(v[q]);
+            if (lane == 0) {
+                sh[q][0][w] = v[q].hi;
+                sh[q][1][w] = v[q].lo;
+            }
+        }
+        __syncthreads();
+        if (w == 0) {
+#pragma unroll
+            for (int q = 0; q < N; q++)
+                v[q] = warp_sum(lane < nw ? kun::DFloat(sh[q][0][lane], sh[q][1][lane]) : kun::DFloat());
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        kun::DFloat r[5];
-        for (int q = 0; q < 5; q++)
-            for (int i = 0; i < kCorrThreads / 32; i++) r[q] = kun::kadd(r[q], kun::DFloat(sh[q][0][i], sh[q][1][i]));
-        // moments in double from the two-float sums: x / S, then the
-        // correlation (XY - X*Y) / (sqrt(X2 - X*X) * sqrt(Y2 - Y*Y))
-        const double n = (double)S;
-        const double mx = ((double)r[0].hi + r[0].lo) / n, my = ((double)r[1].hi + r[1].lo) / n;
-        const double mx2 = ((double)r[2].hi + r[2].lo) / n, my2 = ((double)r[3].hi + r[3].lo) / n;
-        const double mxy = ((double)r[4].hi + r[4].lo) / n;
-        out[k][t] = (float)((mxy - mx * my) / (sqrt(mx2 - mx * mx) * sqrt(my2 - my * my)));
+    static __device__ __forceinline__ kun::DFloat warp_sum(kun::DFloat x) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const kun::DFloat y(__shfl_xor_sync(0xffffffffu, x.hi, o), __shfl_xor_sync(0xffffffffu, x.lo, o));
+            kun::df_acc_pair(x, y);
+            if (!isfinite(x.hi)) x.lo = 0.f;
+        }
+        return x;
     }
+};
+
+// the label row's sum and sum of squares
+__global__ void __launch_bounds__(kCorrThreads) corr_label_rows(const float *__restrict__ y, float4 *__restrict__ ysum,
+                                                                long long S, long long T, int layout, int L) {
+    const long long t = blockIdx.x;
+    CorrSums<2> a;
+    for (long long s = threadIdx.x; s < S; s += blockDim.x) {
+        const float b = y[util_index(layout, s, t, S, T, L)];
+        kun::df_acc(a.v[0], b);
+        kun::df_acc_prod(a.v[1], b, b);
+    }
+    a.reduce(blockDim.x);
+    if (threadIdx.x == 0) ysum[t] = make_float4(a.v[0].hi, a.v[0].lo, a.v[1].hi, a.v[1].lo);
+}
+
+// x, x*x and x*y sums of one (row, input)
+struct CorrRow {
+    float x[2], x2[2], xy[2];
+};
+__device__ __forceinline__ void corr_add(CorrSums<3> &a, float x, float y) {
+    kun::df_acc(a.v[0], x);
+    kun::df_acc_prod(a.v[1], x, x);
+    kun::df_acc_prod(a.v[2], x, y);
+}
+__device__ __forceinline__ void corr_store(const CorrSums<3> &a, CorrRow *o) {
+    *o = CorrRow{{a.v[0].hi, a.v[0].lo}, {a.v[1].hi, a.v[1].lo}, {a.v[2].hi, a.v[2].lo}};
+}
+
+__global__ void __launch_bounds__(kCorrThreads) corr_rows(const float *const *in, const float *__restrict__ y,
+                                                          CorrRow *__restrict__ sums, long long S, long long T,
+                                                          int layout, int L) {
+    const long long t = blockIdx.x;
+    const float *__restrict__ x = in[blockIdx.y];
+    CorrSums<3> a;
+    if (layout == 1) {
+        const float *__restrict__ xr = x + t * S, *__restrict__ yr = y + t * S;
+#pragma unroll 4
+        for (long long s = threadIdx.x; s < S; s += kCorrThreads) corr_add(a, xr[s], yr[s]);
+    } else {
+        for (long long s = threadIdx.x; s < S; s += kCorrThreads) {
+            const long long ix = util_index(layout, s, t, S, T, L);
+            corr_add(a, x[ix], y[ix]);
+        }
+    }
+    a.reduce(kCorrThreads);
+    if (threadIdx.x == 0) corr_store(a, sums + (long long)blockIdx.y * T + t);
+}
+
+// the same with every input row's ranks in place of its values: they are
+// summed where kun::rank_row finds them and never reach memory (5000 stocks x
+// 1250 days x 32 inputs wrote and read 1.6 GB of them, in 33 launches: 5.4 ms,
+// now 2.3 ms, bound by the ranking)
+struct CorrRankAdd {
+    CorrSums<3> &a;
+    const float *__restrict__ y;
+    __device__ __forceinline__ void operator()(int i, float r) const { corr_add(a, r, y[i]); }
+};
+template <int ITEMS, int MAXT>
+__global__ void __launch_bounds__(MAXT, kun::rank_min_blocks<float>(16, MAXT))
+    corr_rank_rows(const float *const *in, const float *__restrict__ y, CorrRow *__restrict__ sums, int S, long long T) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const long long t = blockIdx.x;
+    CorrSums<3> a;
+    kun::rank_row<float, ITEMS>(in[blockIdx.y] + t * S, S, (int)blockDim.x, smem_raw, CorrRankAdd{a, y + t * S});
+    a.reduce(blockDim.x);
+    if (threadIdx.x == 0) corr_store(a, sums + (long long)blockIdx.y * T + t);
+}
+
+// (XY - X*Y) / (sqrt(X2 - X*X) * sqrt(Y2 - Y*Y)) of the means, in double from
+// the two-float sums.  One thread a (row, input): a block's one thread doing
+// it at the end of its row would hold the block for the double divisions.
+__global__ void corr_finish(const CorrRow *__restrict__ sums, const float4 *__restrict__ ysum, float *const *out,
+                            long long S, long long T) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    const CorrRow r = sums[(long long)blockIdx.y * T + t];
+    const float4 q = ysum[t];
+    const double n = (double)S;
+    const double mx = ((double)r.x[0] + r.x[1]) / n, my = ((double)q.x + q.y) / n;
+    const double mx2 = ((double)r.x2[0] + r.x2[1]) / n, my2 = ((double)q.z + q.w) / n;
+    const double mxy = ((double)r.xy[0] + r.xy[1]) / n;
+    out[blockIdx.y][t] = (float)((mxy - mx * my) / (sqrt(mx2 - mx * mx) * sqrt(my2 - my * my)));
 }
 
 // First row of every run of equal consecutive labels (NaN equals nothing), in
@@ -226,34 +298,44 @@ KUN_EXPORT KunStatus kunCorrWith(KunExecutorHandle exec, int n, const float *con
         cudaEventRecord(ex->bridge_in, ex->user_stream);
         cudaStreamWaitEvent(st, ex->bridge_in, 0);
     }
-    const size_t plane = num_stocks * num_time * sizeof(float);
-    // device copies of the pointer arrays (and the ranked planes) in the arena
-    size_t need = 2 * 256 + 2 * (size_t)n * sizeof(void *);
-    if (rank_inputs) need += (size_t)n * ((plane + 255) / 256 * 256);
-    if (!ex->arena.ensure(need)) {
+    if (rank_inputs && num_stocks > (size_t)kun::kRankMaxStocks) {
+        set_error("corrWith: rank failed: %s", cudaGetErrorString(cudaErrorInvalidValue));
+        return KUN_CUDA_ERROR;
+    }
+    // device copies of the pointer arrays and the rows' sums in the arena
+    auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t ptrs = up((size_t)n * sizeof(void *)), ysums = up(num_time * sizeof(float4));
+    if (!ex->arena.ensure(2 * ptrs + ysums + (size_t)n * num_time * sizeof(CorrRow))) {
         set_error("out of device memory for corrWith");
         return KUN_OUT_OF_MEMORY;
     }
     char *base = (char *)ex->arena.ptr;
     const float **d_in = (const float **)base;
-    float **d_out = (float **)(base + (((size_t)n * sizeof(void *) + 255) / 256 * 256));
-    char *ranked = base + 2 * (((size_t)n * sizeof(void *) + 255) / 256 * 256);
-    std::vector<const float *> src(inputs, inputs + n);
-    if (rank_inputs) {
-        for (int k = 0; k < n; k++) {
-            float *r = (float *)(ranked + (size_t)k * ((plane + 255) / 256 * 256));
-            int rc = kun::launch_rank<float>(inputs[k], r, (long long)num_stocks, (long long)num_time, st);
-            if (rc) {
-                set_error("corrWith: rank failed: %s", cudaGetErrorString((cudaError_t)rc));
-                return KUN_CUDA_ERROR;
-            }
-            src[k] = r;
-        }
-    }
-    cudaMemcpyAsync(d_in, src.data(), (size_t)n * sizeof(void *), cudaMemcpyHostToDevice, st);
+    float **d_out = (float **)(base + ptrs);
+    float4 *d_ysum = (float4 *)(base + 2 * ptrs);
+    CorrRow *d_sums = (CorrRow *)(base + 2 * ptrs + ysums);
+    const long long S = (long long)num_stocks, T = (long long)num_time;
+    cudaMemcpyAsync(d_in, inputs, (size_t)n * sizeof(void *), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d_out, outs, (size_t)n * sizeof(void *), cudaMemcpyHostToDevice, st);
-    corr_rows<<<dim3((unsigned)num_time, (unsigned)n), kCorrThreads, 0, st>>>(
-        d_in, corr_with, d_out, (long long)num_stocks, (long long)num_time, layout, 8);
+    corr_label_rows<<<(unsigned)T, kCorrThreads, 0, st>>>(corr_with, d_ysum, S, T, layout, 8);
+    const dim3 grid((unsigned)T, (unsigned)n);
+    if (rank_inputs) {
+        const int rc = kun::rank_dispatch<false>(S, [&](auto items, auto maxt) {
+            constexpr int I = decltype(items)::value, M = decltype(maxt)::value;
+            const int nt = kun::rank_threads((int)S, I);
+            const size_t smem = kun::rank_smem_bytes<float>(nt, I);
+            if (int e = kun::rank_smem_limit(corr_rank_rows<I, M>, smem)) return e;
+            corr_rank_rows<I, M><<<grid, nt, smem, st>>>(d_in, corr_with, d_sums, (int)S, T);
+            return (int)cudaGetLastError();
+        });
+        if (rc) {
+            set_error("corrWith: rank failed: %s", cudaGetErrorString((cudaError_t)rc));
+            return KUN_CUDA_ERROR;
+        }
+    } else {
+        corr_rows<<<grid, kCorrThreads, 0, st>>>(d_in, corr_with, d_sums, S, T, layout, 8);
+    }
+    corr_finish<<<dim3((unsigned)((T + 127) / 128), (unsigned)n), 128, 0, st>>>(d_sums, d_ysum, d_out, S, T);
     if (cudaError_t e = cudaGetLastError()) {
         set_error("corrWith: %s", cudaGetErrorString(e));
         return KUN_CUDA_ERROR;

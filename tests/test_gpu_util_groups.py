@@ -27,3 +27,21 @@ def test_aggregrate_group_edges(dt, T, S, sizes):
     kr.aggregrate(ex, xs, [first, second], got)
     for g, w in zip(got, want):
         assert not compare_exact(g, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S", [2, 31, 128, 129, 997, 4097, 8193])
+@pytest.mark.parametrize("rank", [False, True])
+def test_corrwith_row_lengths(S, rank):
+    rng = np.random.default_rng(S)
+    T = 5
+    xs = [rng.standard_normal((T, S)).astype(np.float32) for _ in range(3)]
+    xs[1] = np.floor(4 * xs[1]) / 4          # ties
+    xs[2][3, 0] = np.nan                     # a NaN row is NaN
+    y = (0.3 * xs[0] + rng.standard_normal((T, S))).astype(np.float32)
+    outs = [np.empty(T, np.float32) for _ in xs]
+    kr.corrWith(kr.createSingleThreadExecutor(), xs, y, outs, rank_inputs=rank)
+    for x, o in zip(xs, outs):
+        # two-float sums: rounding of the float result alone (and of a
+        # correlation of two points, which is 1 or -1)
+        np.testing.assert_allclose(o, U.corr_with(x, y, rank_inputs=rank), rtol=2e-6, atol=2e-6)
