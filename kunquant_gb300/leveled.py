@@ -476,6 +476,8 @@ VEC_U_ELEM = 2
 # rows a window queue loads ahead of use, and the unroll of the window loop
 VEC_PREFETCH = 0
 VEC_UNROLL = 4
+# rows a scan loads while it works on as many others (32 rows are a tenth
+# faster alone, but take 255 registers from the kernels beside it)
 SCAN_BLOCK = 16
 # window sums (two floats each) one chunked scan of the slide form keeps
 SLIDE_MAX_SUMS = 10
@@ -1025,7 +1027,9 @@ class LeveledGen(StageGen):
             # chunked scans have threads enough to hide memory latency; keep
             # the registers for the window sums (single-buffered)
             return SLIDE_BLOCK
-        return SCAN_BLOCK if n <= 6 else (8 if n <= 12 else 4)
+        if any(ops[i]["k"] == "WindowedLinearRegression" for i in role["comp"]):
+            return SCAN_BLOCK // 2
+        return SCAN_BLOCK if n <= 4 else (8 if n <= 8 else 4)
 
     def _scan_prefetch(self, role: dict, B: int, ind: str, chunk: bool = False):
         """Scan role body: rows are processed in blocks of B; every series the
@@ -1050,12 +1054,6 @@ class LeveledGen(StageGen):
         # in a time chunk the scan runs rows [tw, t1) and stores [t0, t1); the
         # rows a state would take out before tw were never put in: NaN
         tbeg, tend, wlo = ("tw", "t1", "tw") if chunk else ("0LL", "length", "0")
-        # double-buffered: the loads of block tb + B are issued before the
-        # state updates of block tb, so memory latency overlaps the scan.
-        # Regression roles compute long enough per row to hide the loads
-        # and keep the registers instead (measured: 478 us single-buffered,
-        # 608 us double-buffered at 2000 stocks)
-        dbl = not any(ops[i]["k"] == "WindowedLinearRegression" for i in comp) and not self.slide
         series = [j for j in sorted(vr) if not (ops[j]["k"] == "Input" and ops[j].get("single_value"))]
         for j in sorted(vr):
             if j not in series:
@@ -1076,22 +1074,16 @@ class LeveledGen(StageGen):
                          f"{pre}{name[1:]}[u] = (r >= {wlo} && {base} + u < {tend}) ? b{src}[r * st{src}] : "
                          f"kun::knan<{T}>(); }}")
 
-        if dbl:
-            for j in series:
-                L.append(f"{ind}{T} pv{j}[{B}], nv{j}[{B}];")
-            for src, off, name in wnames:
-                L.append(f"{ind}{T} {name}[{B}], n{name[1:]}[{B}];")
-            loads("p", tbeg, ind)
+        if not chunk and not self.slide:
+            self._scan_blocks(role, B, ind, series, wnames, wins, stores)
+            return
         L.append(f"{ind}for (long long tb = {tbeg}; tb < {tend}; tb += {B}) {{")
         bi = ind + "  "
-        if dbl:
-            loads("n", f"(tb + {B})", bi)
-        else:
-            for j in series:
-                L.append(f"{bi}{T} pv{j}[{B}];")
-            for src, off, name in wnames:
-                L.append(f"{bi}{T} {name}[{B}];")
-            loads("p", "tb", bi)
+        for j in series:
+            L.append(f"{bi}{T} pv{j}[{B}];")
+        for src, off, name in wnames:
+            L.append(f"{bi}{T} {name}[{B}];")
+        loads("p", "tb", bi)
         L.append(f"{bi}#pragma unroll")
         L.append(f"{bi}for (int u = 0; u < {B}; ++u) {{")
         bj = bi + "  "
@@ -1125,12 +1117,76 @@ class LeveledGen(StageGen):
         for i in stores:
             L.append(f"{bj}{guard}b{i}[t * st{i}] = {self.val(i)};")
         L.append(f"{bi}}}")
-        for j in series if dbl else []:
+        L.append(f"{ind}}}")
+
+    def _scan_blocks(self, role: dict, B: int, ind: str, series: List[int], wnames, wins, stores: List[int]):
+        """The rows of a whole scan in blocks of B, the next block's loads
+        issued before the states step through the present one.  A block's
+        loads and steps are straight-line code: rows are tested only in a
+        load block that touches the ends and in the last, partial block of
+        steps (a test a row cuts the steps apart, and the rows' independent
+        parts no longer overlap: 68 us against 36 for five 60-row sums of 997
+        stocks x 1251 days, 174 against 152 at 5000 x 2500)."""
+        ops, T, L = self.ops, self.T, self.lines
+        comp, vr = role["comp"], role["vr"]
+        tag = role["roots"][0]
+        arrays = [f"v{j}" for j in series] + [name[1:] for _, _, name in wnames]
+        wmax = max([int(off) for _, off, _ in wnames] + [0])
+        for x in arrays:
+            L.append(f"{ind}{T} p{x}[{B}], n{x}[{B}];")
+        params = "".join(f"{T} (&a{x})[{B}], " for x in arrays)
+        L.append(f"{ind}auto load{tag} = [&]({params}const long long tl) {{")
+        bi, bj = ind + "  ", ind + "    "
+        L.append(f"{bi}if (tl >= {wmax} && tl + {B} <= length) {{")
+        for j in series:
+            L.append(f"{bj}#pragma unroll")
+            L.append(f"{bj}for (int u = 0; u < {B}; ++u) av{j}[u] = b{j}[(tl + u) * st{j}];")
+        for src, off, name in wnames:
+            L.append(f"{bj}#pragma unroll")
+            L.append(f"{bj}for (int u = 0; u < {B}; ++u) a{name[1:]}[u] = b{src}[(tl + u - {off}) * st{src}];")
+        L.append(f"{bi}}} else {{")
+        for j in series:
+            L.append(f"{bj}#pragma unroll")
+            L.append(f"{bj}for (int u = 0; u < {B}; ++u) av{j}[u] = tl + u < length ? b{j}[(tl + u) * st{j}] : "
+                     f"kun::knan<{T}>();")
+        for src, off, name in wnames:
+            L.append(f"{bj}#pragma unroll")
+            L.append(f"{bj}for (int u = 0; u < {B}; ++u) a{name[1:]}[u] = (tl + u >= {off} && tl + u < length) ? "
+                     f"b{src}[(tl + u - {off}) * st{src}] : kun::knan<{T}>();")
+        L.append(f"{bi}}}")
+        L.append(f"{ind}}};")
+
+        def args(pre):
+            return "".join(f"{pre}{x}, " for x in arrays)
+
+        def steps(guard):
             L.append(f"{bi}#pragma unroll")
-            L.append(f"{bi}for (int u = 0; u < {B}; ++u) pv{j}[u] = nv{j}[u];")
-        for src, off, name in wnames if dbl else []:
+            L.append(f"{bi}for (int u = 0; u < {B}; ++u) {{")
+            L.append(f"{bj}const long long t = tb + u;")
+            if guard:
+                L.append(f"{bj}if (t >= length) break;")
+            for j in sorted(vr):
+                L.append(f"{bj}const {T} v{j} = pv{j}" + (";" if j not in series else "[u];"))
+            self.pf_window = wins
+            for i in range(len(ops)):
+                if i in comp and ops[i].get("p", -1) < 0:
+                    self.emit_top(i, bj, {}, comp)
+            self.pf_window = None
+            for i in stores:
+                L.append(f"{bj}b{i}[t * st{i}] = {self.val(i)};")
+            L.append(f"{bi}}}")
+
+        L.append(f"{ind}long long tb = 0;")
+        L.append(f"{ind}load{tag}({args('p')}0);")
+        L.append(f"{ind}for (; tb + {B} <= length; tb += {B}) {{")
+        L.append(f"{bi}load{tag}({args('n')}tb + {B});")
+        steps(False)
+        for x in arrays:
             L.append(f"{bi}#pragma unroll")
-            L.append(f"{bi}for (int u = 0; u < {B}; ++u) {name}[u] = n{name[1:]}[u];")
+            L.append(f"{bi}for (int u = 0; u < {B}; ++u) p{x}[u] = n{x}[u];")
+        L.append(f"{ind}}}")
+        L.append(f"{ind}if (tb < length) {{")
+        steps(True)
         L.append(f"{ind}}}")
 
     # ------------------------------------------------------------------ staged (TMA) form
