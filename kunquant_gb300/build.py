@@ -74,7 +74,7 @@ def runtime_path() -> str:
 
 def build_runtime(force: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    srcs = [os.path.join(CSRC, f) for f in ("kun_runtime.cu", "kun_stream.cu", "kun_serve.cu", "kun_batch.cu",
+    srcs = [os.path.join(CSRC, f) for f in ("kun_runtime.cu", "kun_plan.cu", "kun_stream.cu", "kun_serve.cu", "kun_batch.cu",
                                             "kun_util.cu", "kun_noalloc.cu")]
     srcs = [s for s in srcs if os.path.exists(s)]
     lib = runtime_path()

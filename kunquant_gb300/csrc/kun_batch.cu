@@ -6,8 +6,10 @@
 // ONCE over the tiles of all jobs (the job of a block is found from a tile
 // table passed by value); a Rank stage ranks every job's rows in one launch;
 // other stages run job by job.  The jobs' parameter
-// blocks go to the device with one copy per stage.  This replaces the
-// reference's one runGraph per universe (cpp/Kun/Runtime.cpp:311-352).
+// blocks go to the device with one copy per stage.  On an executor of several
+// streams the kernels of all stages run as one graph of nodes (kun_plan.cu)
+// after one copy of all blocks.  This replaces the reference's one runGraph per
+// universe (cpp/Kun/Runtime.cpp:311-352).
 //
 // kunExecutorTune picks, per stage, the time tile of the time-parallel
 // kernels and the threads per block by timing candidate shapes on the jobs
@@ -40,7 +42,7 @@ struct BatchJob {
     long long S, total_time, cur_time, length;
     const Plan *plan;
     std::vector<void *> ptrs;
-    size_t arena_off;
+    size_t arena_off, slot_bytes;
 };
 
 struct BatchRun {
@@ -48,12 +50,38 @@ struct BatchRun {
     const KunGpuModuleDesc *m;
     std::vector<BatchJob> jobs;
     std::vector<int> order;
-    size_t host_off = 0;  // parameter blocks staged so far in this run
+    const Plan *nodes = nullptr;  // the jobs' common plan in kernels, or null: stage by stage
+    size_t host_off = 0;          // parameter blocks staged so far in this run
 };
+
+// The plan in kernels that all jobs share on a multi-stream executor: slots
+// are numbered alike in every job's part of the arena, and the kernels are
+// weighed by the jobs' summed cells.  Null when the module or memory has none.
+static const Plan *batch_node_plan(Executor *ex, const KunGpuModuleDesc *m, const std::vector<BatchJob> &jobs) {
+    const int ns = (int)ex->streams.size();
+    if (ns < 2 || jobs.size() < 2) return nullptr;
+    long long cells = 0, rows = 0;
+    size_t slot_bytes = 0;
+    for (const BatchJob &jb : jobs) {
+        cells += jb.S * jb.length;
+        rows = std::max(rows, jb.length);
+        slot_bytes += jb.slot_bytes;
+    }
+    auto key = std::make_tuple((const void *)m, -cells, -rows, ns);  // negative: not a single run's
+    auto it = ex->plans.find(key);
+    if (it == ex->plans.end()) {
+        Plan p;
+        if (!make_plan(m, jobs[0].S, jobs[0].length, ns, p)) return nullptr;
+        p.slot_bytes = slot_bytes;
+        make_node_plan(m, (double)cells, (double)rows, ns, node_slots(p), p);
+        it = ex->plans.emplace(key, std::move(p)).first;
+    }
+    return it->second.nodes.empty() ? nullptr : &it->second;
+}
 
 static KunStatus batch_setup(Executor *ex, const KunGpuModuleDesc *m, int njobs, const NameMap *const *maps,
                              const size_t *S, const size_t *total_time, const size_t *cur_time,
-                             const size_t *length, BatchRun &br) {
+                             const size_t *length, bool by_kernel, BatchRun &br) {
     if (!ex || !m || njobs <= 0 || !maps || !S || !total_time || !cur_time || !length) {
         set_error("kunRunGraphBatch: bad arguments");
         return KUN_INVALID_ARGUMENT;
@@ -92,11 +120,20 @@ static KunStatus batch_setup(Executor *ex, const KunGpuModuleDesc *m, int njobs,
             it = ex->plans.emplace(key, std::move(p)).first;
         }
         jb.plan = &it->second;
-        jb.arena_off = total;
-        total += (jb.plan->slot_bytes * (size_t)jb.plan->num_slots + 255) / 256 * 256;
+        jb.slot_bytes = jb.plan->slot_bytes;
     }
     br.order = br.jobs[0].plan->order;
-    if (!ex->arena.ensure(total)) {
+    if (by_kernel && (br.nodes = batch_node_plan(ex, m, br.jobs)))
+        for (BatchJob &jb : br.jobs) jb.plan = br.nodes;
+    for (BatchJob &jb : br.jobs) {
+        jb.arena_off = total;
+        total += (jb.slot_bytes * (size_t)jb.plan->num_slots + 255) / 256 * 256;
+    }
+    if (!ex->arena.ensure(total) && br.nodes) {  // the plan in stages may need less
+        br = BatchRun();
+        return batch_setup(ex, m, njobs, maps, S, total_time, cur_time, length, false, br);
+    }
+    if (ex->arena.bytes < total) {
         set_error("out of device memory for the temporaries of %d jobs (%zu bytes)", njobs, total);
         return KUN_OUT_OF_MEMORY;
     }
@@ -108,7 +145,7 @@ static KunStatus batch_setup(Executor *ex, const KunGpuModuleDesc *m, int njobs,
             if (bd.kind == KUN_BUF_TEMP) {
                 if (jb.plan->temp_slot[b] >= 0)
                     jb.ptrs[b] = (char *)ex->arena.ptr + jb.arena_off +
-                                 jb.plan->slot_bytes * (size_t)jb.plan->temp_slot[b];
+                                 jb.slot_bytes * (size_t)jb.plan->temp_slot[b];
                 continue;
             }
             auto f = maps[j]->find(bd.name);
@@ -139,24 +176,33 @@ static bool ensure_group_staging(Executor *ex, size_t need) {
     return ex->group_dev.ensure(need);
 }
 
-// Enqueue stage `si` for every job; `tile`/`block` override the tuning table.
-static KunStatus batch_stage(BatchRun &br, int si, cudaStream_t st, const int32_t *tile, const int32_t *block,
-                             int64_t &launches) {
+// One stage's launch arguments for every job, and its parameter blocks (or
+// the grouped Rank's job table) in the pinned staging.
+struct StageBlocks {
+    std::vector<std::vector<void *>> scratch;
+    std::vector<KunGpuStageArgs> args;
+    std::vector<size_t> off;  // per group of KUN_GROUP_MAX jobs
+    bool rank = false;
+    int rank_jobs = 0;
+    long long rank_rows = 0, rank_max = 0;
+};
+
+static KunStatus stage_blocks(BatchRun &br, int si, const int32_t *tile, const int32_t *block, StageBlocks &sb) {
     Executor *ex = br.ex;
     const KunGpuModuleDesc *m = br.m;
     const KunGpuStageDesc &d = m->stages[si];
     const int n = (int)br.jobs.size();
-    std::vector<std::vector<void *>> scratch(n);
-    std::vector<KunGpuStageArgs> args(n);
+    sb.scratch.resize(n);
+    sb.args.resize(n);
     auto tn = ex->tuning.find((const void *)m);
     for (int j = 0; j < n; j++) {
         BatchJob &jb = br.jobs[j];
         for (int sl : jb.plan->scratch[si])
-            scratch[j].push_back((char *)ex->arena.ptr + jb.arena_off + jb.plan->slot_bytes * (size_t)sl);
-        KunGpuStageArgs &a = args[j];
+            sb.scratch[j].push_back((char *)ex->arena.ptr + jb.arena_off + jb.slot_bytes * (size_t)sl);
+        KunGpuStageArgs &a = sb.args[j];
         memset(&a, 0, sizeof a);
         a.buffers = jb.ptrs.data();
-        a.scratch = scratch[j].data();
+        a.scratch = sb.scratch[j].data();
         a.num_stocks = jb.S;
         a.total_time = jb.total_time;
         a.start = jb.cur_time;
@@ -170,15 +216,24 @@ static KunStatus batch_stage(BatchRun &br, int si, cudaStream_t st, const int32_
             a.tune_block = tn->second[si].block.data();
         }
     }
+    auto stage_room = [&](size_t bytes) {
+        const size_t off = (br.host_off + 255) / 256 * 256;
+        if (off + bytes > ex->group_host_bytes) {
+            set_error("grouped launch staging exhausted");
+            return false;
+        }
+        sb.off.push_back(off);
+        br.host_off = off + bytes;
+        return true;
+    };
     // Rank stages in the TS layout: every job's rows in one launch
-    const bool ts_rank = d.kind == KUN_STAGE_RANK && n > 1 && d.num_in == 1 && d.num_out == 1 &&
-                         (m->buffers[d.in_bufs[0]].kind != KUN_BUF_INPUT || m->input_layout == KUN_LAYOUT_TS) &&
-                         (m->buffers[d.out_bufs[0]].kind != KUN_BUF_OUTPUT || m->output_layout == KUN_LAYOUT_TS);
-    if (ts_rank) {
+    sb.rank = d.kind == KUN_STAGE_RANK && n > 1 && d.num_in == 1 && d.num_out == 1 &&
+              (m->buffers[d.in_bufs[0]].kind != KUN_BUF_INPUT || m->input_layout == KUN_LAYOUT_TS) &&
+              (m->buffers[d.out_bufs[0]].kind != KUN_BUF_OUTPUT || m->output_layout == KUN_LAYOUT_TS);
+    if (sb.rank) {
         const int bi = d.in_bufs[0], bo = d.out_bufs[0];
         const size_t esz = m->dtype == 0 ? 4 : 8;
         std::vector<kun::RankRowsJob> jobs;
-        long long rows = 0, max_S = 0;
         for (int j = 0; j < n; j++) {
             const BatchJob &jb = br.jobs[j];
             if (jb.S <= 0 || jb.length <= 0) continue;
@@ -188,64 +243,95 @@ static KunStatus batch_stage(BatchRun &br, int si, cudaStream_t st, const int32_
             rj.out = jb.ptrs[bo];
             rj.S = jb.S;
             rj.length = jb.length;
-            rj.row0 = rows;
-            rows += jb.length;
-            max_S = std::max(max_S, jb.S);
+            rj.row0 = sb.rank_rows;
+            sb.rank_rows += jb.length;
+            sb.rank_max = std::max(sb.rank_max, jb.S);
             jobs.push_back(rj);
         }
-        const size_t bytes = jobs.size() * sizeof(kun::RankRowsJob);
-        const size_t off = (br.host_off + 255) / 256 * 256;
-        if (off + bytes > ex->group_host_bytes) {
-            set_error("grouped launch staging exhausted");
-            return KUN_OUT_OF_MEMORY;
+        sb.rank_jobs = (int)jobs.size();
+        if (!stage_room(jobs.size() * sizeof(kun::RankRowsJob))) return KUN_OUT_OF_MEMORY;
+        memcpy((char *)ex->group_host + sb.off[0], jobs.data(), jobs.size() * sizeof(kun::RankRowsJob));
+    } else if (d.launch_group && n > 1) {
+        for (int j0 = 0; j0 < n; j0 += KUN_GROUP_MAX) {
+            const int nj = std::min(KUN_GROUP_MAX, n - j0);
+            if (!stage_room(d.prepare(&sb.args[j0], nj, nullptr))) return KUN_OUT_OF_MEMORY;
+            d.prepare(&sb.args[j0], nj, (char *)ex->group_host + sb.off.back());
         }
-        memcpy((char *)ex->group_host + off, jobs.data(), bytes);
-        char *dev = (char *)ex->group_dev.ptr + off;
-        cudaMemcpyAsync(dev, (char *)ex->group_host + off, bytes, cudaMemcpyHostToDevice, st);
-        int rc = m->dtype == 0 ? kun::launch_rank_rows_multi<float>((const kun::RankRowsJob *)dev, (int)jobs.size(),
-                                                                    rows, max_S, st)
-                               : kun::launch_rank_rows_multi<double>((const kun::RankRowsJob *)dev,
-                                                                     (int)jobs.size(), rows, max_S, st);
-        if (rc) {
-            set_error("stage %d (%s) grouped Rank failed: %s", si, d.name, cudaGetErrorString((cudaError_t)rc));
-            return KUN_CUDA_ERROR;
-        }
-        br.host_off = off + bytes;
+    }
+    return KUN_SUCCESS;
+}
+
+// Launches a stage (kernel < 0) or one of its kernels, its blocks on the device
+static KunStatus launch_blocks(BatchRun &br, int si, int kernel, StageBlocks &sb, cudaStream_t st, int64_t &launches) {
+    const KunGpuModuleDesc *m = br.m;
+    const KunGpuStageDesc &d = m->stages[si];
+    const int n = (int)br.jobs.size();
+    char *dev = (char *)br.ex->group_dev.ptr;
+    const int kernels = kernel >= 0 || d.num_kernels <= 0 ? 1 : d.num_kernels;
+    auto failed = [&](const char *what, int rc) {
+        set_error("stage %d (%s) %s failed: %s", si, d.name, what, cudaGetErrorString((cudaError_t)rc));
+        return KUN_CUDA_ERROR;
+    };
+    if (sb.rank) {
+        const auto *jobs = (const kun::RankRowsJob *)(dev + sb.off[0]);
+        int rc = m->dtype == 0
+                     ? kun::launch_rank_rows_multi<float>(jobs, sb.rank_jobs, sb.rank_rows, sb.rank_max, st)
+                     : kun::launch_rank_rows_multi<double>(jobs, sb.rank_jobs, sb.rank_rows, sb.rank_max, st);
+        if (rc) return failed("grouped Rank", rc);
         launches += 1;
         return KUN_SUCCESS;
     }
-    if (d.launch_group && n > 1) {
-        for (int j0 = 0; j0 < n; j0 += KUN_GROUP_MAX) {
-            const int nj = std::min(KUN_GROUP_MAX, n - j0);
-            const size_t bytes = d.prepare(&args[j0], nj, nullptr);
-            const size_t off = (br.host_off + 255) / 256 * 256;
-            if (off + bytes > ex->group_host_bytes) {
-                set_error("grouped launch staging exhausted");
-                return KUN_OUT_OF_MEMORY;
-            }
-            d.prepare(&args[j0], nj, (char *)ex->group_host + off);
-            char *dev = (char *)ex->group_dev.ptr + off;
-            cudaMemcpyAsync(dev, (char *)ex->group_host + off, bytes, cudaMemcpyHostToDevice, st);
-            int rc = d.launch_group(&args[j0], nj, dev, (void *)st);
-            if (rc) {
-                set_error("stage %d (%s) grouped launch failed: %s", si, d.name, cudaGetErrorString((cudaError_t)rc));
-                return KUN_CUDA_ERROR;
-            }
-            br.host_off = off + bytes;
-            launches += d.num_kernels > 0 ? d.num_kernels : 1;
+    for (KunGpuStageArgs &a : sb.args) a.only_kernel = kernel + 1;
+    if (!sb.off.empty()) {
+        for (size_t g = 0; g < sb.off.size(); g++) {
+            const int j0 = (int)g * KUN_GROUP_MAX;
+            if (int rc = d.launch_group(&sb.args[j0], std::min(KUN_GROUP_MAX, n - j0), dev + sb.off[g], (void *)st))
+                return failed("grouped launch", rc);
+            launches += kernels;
         }
         return KUN_SUCCESS;
     }
     for (int j = 0; j < n; j++) {
-        int rc = d.launch(&args[j], (void *)st);
-        if (rc) {
+        if (int rc = d.launch(&sb.args[j], (void *)st)) {
             set_error("stage %d (%s) launch failed for job %d: %s", si, d.name, j,
                       cudaGetErrorString((cudaError_t)rc));
             return KUN_CUDA_ERROR;
         }
-        launches += d.num_kernels > 0 ? d.num_kernels : 1;
+        launches += kernels;
     }
     return KUN_SUCCESS;
+}
+
+static void copy_blocks(BatchRun &br, size_t from, cudaStream_t st) {
+    if (br.host_off > from)
+        cudaMemcpyAsync((char *)br.ex->group_dev.ptr + from, (char *)br.ex->group_host + from, br.host_off - from,
+                        cudaMemcpyHostToDevice, st);
+}
+
+// Enqueue stage `si` for every job; `tile`/`block` override the tuning table.
+static KunStatus batch_stage(BatchRun &br, int si, cudaStream_t st, const int32_t *tile, const int32_t *block,
+                             int64_t &launches) {
+    StageBlocks sb;
+    const size_t from = br.host_off;
+    KunStatus rs = stage_blocks(br, si, tile, block, sb);
+    if (rs != KUN_SUCCESS) return rs;
+    copy_blocks(br, from, st);
+    return launch_blocks(br, si, -1, sb, st, launches);
+}
+
+// Every kernel of the module on the executor's streams: all parameter blocks
+// go to the device in one copy, then each kernel runs once over all jobs as
+// soon as what it reads is there.
+static KunStatus batch_nodes(BatchRun &br, cudaStream_t st, int64_t &launches) {
+    std::vector<StageBlocks> blocks(br.m->num_stages);
+    KunStatus rs = KUN_SUCCESS;
+    for (int si : br.order)
+        if ((rs = stage_blocks(br, si, nullptr, nullptr, blocks[si])) != KUN_SUCCESS) return rs;
+    copy_blocks(br, 0, st);
+    run_nodes(br.ex, *br.nodes, st, [&](int, const PlanNode &n, cudaStream_t on) {
+        return (rs = launch_blocks(br, n.stage, n.kernel, blocks[n.stage], on, launches)) == KUN_SUCCESS;
+    });
+    return rs;
 }
 
 // bytes of the parameter blocks of one pass over all stages
@@ -307,7 +393,7 @@ KUN_EXPORT KunStatus kunRunGraphBatch(KunExecutorHandle exec, KunModuleHandle mo
     ex->check_epoch();
     BatchRun br;
     KunStatus rs = batch_setup(ex, (const KunGpuModuleDesc *)mod, njobs, (const NameMap *const *)buffers,
-                               num_stocks, total_time, cur_time, length, br);
+                               num_stocks, total_time, cur_time, length, !ex->profile, br);
     if (rs != KUN_SUCCESS) return rs;
     if ((rs = batch_begin(ex, br, 1)) != KUN_SUCCESS) return rs;
     cudaStream_t st = ex->stream();
@@ -316,8 +402,14 @@ KUN_EXPORT KunStatus kunRunGraphBatch(KunExecutorHandle exec, KunModuleHandle mo
         cudaStreamWaitEvent(st, ex->bridge_in, 0);
     }
     int64_t launches = 0;
+    if (br.nodes) {
+        if ((rs = batch_nodes(br, st, launches)) != KUN_SUCCESS) {
+            for (cudaStream_t q : ex->streams) cudaStreamSynchronize(q);  // kernels enqueued so far use the buffers
+            return rs;
+        }
+    }
     for (int si : br.order)
-        if ((rs = batch_stage(br, si, st, nullptr, nullptr, launches)) != KUN_SUCCESS) return rs;
+        if (!br.nodes && (rs = batch_stage(br, si, st, nullptr, nullptr, launches)) != KUN_SUCCESS) return rs;
     ex->last_launches = launches;
     return batch_finish(ex, st, synchronize != 0);
 }
@@ -341,8 +433,8 @@ KUN_EXPORT int kunExecutorTune(KunExecutorHandle exec, KunModuleHandle mod, int 
     ex->check_epoch();
     const auto *m = (const KunGpuModuleDesc *)mod;
     BatchRun br;
-    if (batch_setup(ex, m, njobs, (const NameMap *const *)buffers, num_stocks, total_time, cur_time, length, br) !=
-        KUN_SUCCESS)
+    if (batch_setup(ex, m, njobs, (const NameMap *const *)buffers, num_stocks, total_time, cur_time, length, false,
+                    br) != KUN_SUCCESS)
         return -1;
     reps = std::max(1, reps);
     const int tiles[] = {0, 16, 32, 64, 128, 256};

@@ -11,7 +11,7 @@
 extern "C" {
 #endif
 
-#define KUN_GPU_MODULE_ABI 0x6b470009ull
+#define KUN_GPU_MODULE_ABI 0x6b47000aull
 #define KUN_BLOCK_REGCAP 0x10000
 
 typedef enum { KUN_LAYOUT_STS = 0, KUN_LAYOUT_TS = 1, KUN_LAYOUT_STREAM = 2 } KunGpuLayout;
@@ -67,6 +67,9 @@ typedef struct {
      * time-parallel kernel's instance compiled for 64 registers a thread */
     const int32_t *tune_tile;
     const int32_t *tune_block;
+    /* stages with kernel_info: 0 launches every kernel of the stage in order,
+     * k + 1 its kernel k alone (grouped launches read it from args[0]) */
+    int32_t only_kernel;
 } KunGpuStageArgs;
 
 typedef int (*KunGpuLaunchFn)(const KunGpuStageArgs *args, void *cuda_stream);
@@ -102,7 +105,11 @@ typedef struct {
      * kernel reads them.  NULL when state_i_vars is 0. */
     const int32_t *state_i_max;
     /* time-series stages with grouped launches: per kernel, default time
-     * tile << 1 (or number of scan roles << 1) | 1 for a scan kernel */
+     * tile << 1 (or number of scan roles << 1) | 1 for a scan kernel.  Behind
+     * these num_kernels entries, per kernel: the instructions a cell takes
+     * (an estimate), the number of series it reads from other kernels and
+     * those, the number it writes and those; a series is a buffer id, or
+     * -1 - k for the stage's scratch k */
     const int32_t *kernel_info;
     KunGpuPrepareFn prepare;
     KunGpuGroupLaunchFn launch_group;

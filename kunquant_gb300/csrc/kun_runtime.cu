@@ -209,14 +209,14 @@ struct OutputCopies {
         const void *dev;
         size_t bytes;
     };
-    std::vector<std::vector<Item>> by_stage;  // stage -> outputs it produces
+    std::vector<std::vector<Item>> by_step;  // stage, or node of the plan -> outputs it produces
     int next = 0;
 };
 
-static void issue_stage_copies(Executor *ex, OutputCopies &oc, int si, cudaStream_t st) {
-    auto &items = oc.by_stage[si];
+static void issue_copies(Executor *ex, OutputCopies &oc, int step, cudaStream_t st) {
+    auto &items = oc.by_step[step];
     if (items.empty()) return;
-    cudaEvent_t ev = ex->copy_ev[si];
+    cudaEvent_t ev = ex->copy_ev[step];
     cudaEventRecord(ev, st);
     for (auto &it : items) {
         cudaStream_t cs = ex->copy_streams[oc.next++ % ex->copy_streams.size()];
@@ -225,10 +225,80 @@ static void issue_stage_copies(Executor *ex, OutputCopies &oc, int si, cudaStrea
     }
 }
 
+// the arguments of one stage's launches
+static KunGpuStageArgs stage_args(Executor *ex, const KunGpuModuleDesc *m, const Plan &plan, int si, void **ptrs,
+                                  std::vector<void *> &scratch, long long S, long long total_time,
+                                  long long cur_time, long long length) {
+    scratch.clear();
+    for (int sl : plan.scratch[si]) scratch.push_back((char *)ex->arena.ptr + plan.slot_bytes * (size_t)sl);
+    KunGpuStageArgs a;
+    memset(&a, 0, sizeof a);
+    a.buffers = ptrs;
+    a.scratch = scratch.data();
+    a.num_stocks = S;
+    a.total_time = total_time;
+    a.start = cur_time;
+    a.length = length;
+    a.error_flag = ex->d_error;
+    auto tn = ex->tuning.find((const void *)m);
+    if (tn != ex->tuning.end() && si < (int)tn->second.size() && !tn->second[si].tile.empty()) {
+        a.tune_tile = tn->second[si].tile.data();
+        a.tune_block = tn->second[si].block.data();
+    }
+    return a;
+}
+
+KunStatus fork_streams(Executor *ex, int num_streams, cudaStream_t origin) {
+    if (!ex->fork) cudaEventCreateWithFlags(&ex->fork, cudaEventDisableTiming);
+    cudaEventRecord(ex->fork, origin);
+    for (int k = 1; k < num_streams; k++)
+        if (ex->streams[k] != origin) cudaStreamWaitEvent(ex->streams[k], ex->fork, 0);
+    return KUN_SUCCESS;
+}
+
+void run_nodes(Executor *ex, const Plan &plan, cudaStream_t origin,
+               const std::function<bool(int, const PlanNode &, cudaStream_t)> &launch) {
+    ensure_events(ex->done, plan.nodes.size(), cudaEventDisableTiming);
+    fork_streams(ex, plan.num_streams, origin);
+    std::vector<int> last(plan.num_streams, -1);
+    for (int i = 0; i < (int)plan.nodes.size(); i++) {
+        const PlanNode &n = plan.nodes[i];
+        cudaStream_t st = n.stream == 0 ? origin : ex->streams[n.stream];
+        for (int w : n.waits) cudaStreamWaitEvent(st, ex->done[w], 0);
+        if (!launch(i, n, st)) return;
+        if (n.signal) cudaEventRecord(ex->done[i], st);
+        last[n.stream] = i;
+    }
+    for (int k = 1; k < plan.num_streams; k++) {
+        if (last[k] < 0) continue;
+        if (!plan.nodes[last[k]].signal) cudaEventRecord(ex->done[last[k]], ex->streams[k]);
+        cudaStreamWaitEvent(origin, ex->done[last[k]], 0);
+    }
+}
+
 static KunStatus enqueue_stages(Executor *ex, const KunGpuModuleDesc *m, const Plan &plan, void **ptrs,
                                 long long S, long long total_time, long long cur_time, long long length,
                                 cudaStream_t origin, bool multi, int64_t &launches, OutputCopies *oc = nullptr) {
     std::vector<void *> scratch;
+    auto fail = [&](int si, int rc) {
+        set_error("stage %d (%s) launch failed: %s", si, m->stages[si].name, cudaGetErrorString((cudaError_t)rc));
+        return KUN_CUDA_ERROR;
+    };
+    if (multi && !plan.nodes.empty()) {
+        KunStatus rs = KUN_SUCCESS;
+        run_nodes(ex, plan, origin, [&](int i, const PlanNode &n, cudaStream_t st) {
+            KunGpuStageArgs a = stage_args(ex, m, plan, n.stage, ptrs, scratch, S, total_time, cur_time, length);
+            a.only_kernel = n.kernel + 1;
+            if (int rc = m->stages[n.stage].launch(&a, (void *)st)) {
+                rs = fail(n.stage, rc);
+                return false;
+            }
+            launches += n.kernel >= 0 || m->stages[n.stage].num_kernels <= 0 ? 1 : m->stages[n.stage].num_kernels;
+            if (oc) issue_copies(ex, *oc, i, st);
+            return true;
+        });
+        return rs;
+    }
     int ev_idx = 0;
     if (ex->profile) {
         ensure_events(ex->ev, plan.order.size() + 1, cudaEventDefault);
@@ -237,10 +307,7 @@ static KunStatus enqueue_stages(Executor *ex, const KunGpuModuleDesc *m, const P
     }
     if (multi) {
         ensure_events(ex->done, m->num_stages, cudaEventDisableTiming);
-        if (!ex->fork) cudaEventCreateWithFlags(&ex->fork, cudaEventDisableTiming);
-        cudaEventRecord(ex->fork, origin);
-        for (int k = 0; k < plan.num_streams; k++)
-            if (ex->streams[k] != origin) cudaStreamWaitEvent(ex->streams[k], ex->fork, 0);
+        fork_streams(ex, plan.num_streams, origin);
     }
     std::vector<int> last_on(plan.num_streams, -1);
     for (int si : plan.order) {
@@ -252,30 +319,12 @@ static KunStatus enqueue_stages(Executor *ex, const KunGpuModuleDesc *m, const P
             for (int d : plan.preds[si])
                 if (plan.stream_of[d] != k) cudaStreamWaitEvent(st, ex->done[d], 0);
         }
-        scratch.clear();
-        for (int sl : plan.scratch[si]) scratch.push_back((char *)ex->arena.ptr + plan.slot_bytes * (size_t)sl);
-        KunGpuStageArgs a;
-        memset(&a, 0, sizeof a);
-        a.buffers = ptrs;
-        a.scratch = scratch.data();
-        a.num_stocks = S;
-        a.total_time = total_time;
-        a.start = cur_time;
-        a.length = length;
-        a.error_flag = ex->d_error;
-        auto tn = ex->tuning.find((const void *)m);
-        if (tn != ex->tuning.end() && si < (int)tn->second.size() && !tn->second[si].tile.empty()) {
-            a.tune_tile = tn->second[si].tile.data();
-            a.tune_block = tn->second[si].block.data();
-        }
+        KunGpuStageArgs a = stage_args(ex, m, plan, si, ptrs, scratch, S, total_time, cur_time, length);
         int rc = s.launch(&a, (void *)st);
         launches += s.num_kernels > 0 ? s.num_kernels : 1;
-        if (rc != 0) {
-            set_error("stage %d (%s) launch failed: %s", si, s.name, cudaGetErrorString((cudaError_t)rc));
-            return KUN_CUDA_ERROR;
-        }
+        if (rc != 0) return fail(si, rc);
         if (ex->profile) cudaEventRecord(ex->ev[++ev_idx], st);
-        if (oc) issue_stage_copies(ex, *oc, si, st);
+        if (oc) issue_copies(ex, *oc, si, st);
         if (multi) {
             cudaEventRecord(ex->done[si], st);
             last_on[plan.stream_of[si]] = si;
@@ -300,6 +349,19 @@ void Executor::check_epoch() {
     plans.clear();
     tuning.clear();
     epoch = e;
+}
+
+// Slots a plan in kernels may take where the plan in stages takes num_slots:
+// more kernels are live at once, so somewhat more, and never so much that a
+// run that fitted beside the caller's tensors no longer does.
+int node_slots(const Plan &p) {
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return p.num_slots;
+    }
+    const size_t spare = free_bytes / 16 / std::max<size_t>(1, p.slot_bytes);
+    return p.num_slots + (int)std::min<size_t>(spare, (size_t)p.num_slots);
 }
 
 KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &names, long long S,
@@ -338,11 +400,17 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
     if (it == ex->plans.end()) {
         Plan p;
         if (!make_plan(m, S, length, nstreams, p)) return KUN_INVALID_ARGUMENT;
+        if (multi) make_node_plan(m, (double)S * (double)length, (double)length, nstreams, node_slots(p), p);
         it = ex->plans.emplace(key, std::move(p)).first;
     }
     const Plan &plan = it->second;
     size_t elem = m->dtype == 0 ? 4 : 8;
-    if (!ex->arena.ensure(plan.slot_bytes * (size_t)plan.num_slots)) {
+    auto arena_fits = [&] { return ex->arena.ensure(plan.slot_bytes * (size_t)plan.num_slots); };
+    if (!arena_fits() && !plan.nodes.empty()) {  // the plan in stages may need less
+        it->second = Plan();
+        if (!make_plan(m, S, length, nstreams, it->second)) return KUN_INVALID_ARGUMENT;
+    }
+    if (!arena_fits()) {
         set_error("out of device memory for %d temporaries of %zu bytes", plan.num_slots, plan.slot_bytes);
         return KUN_OUT_OF_MEMORY;
     }
@@ -423,18 +491,22 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
         }
     }
     if (overlap) {
-        ensure_events(ex->copy_ev, m->num_stages, cudaEventDisableTiming);
+        const bool by_node = multi && !plan.nodes.empty();
+        const size_t steps = by_node ? plan.nodes.size() : (size_t)m->num_stages;
+        ensure_events(ex->copy_ev, steps, cudaEventDisableTiming);
         ensure_events(ex->copy_done, ex->copy_streams.size(), cudaEventDisableTiming);
-        oc.by_stage.assign(m->num_stages, {});
+        oc.by_step.assign(steps, {});
         std::vector<int> producer(m->num_buffers, -1);
-        for (int si = 0; si < m->num_stages; si++)
+        for (int i = 0; by_node && i < (int)steps; i++)
+            for (int b : plan.nodes[i].outs) producer[b] = i;
+        for (int si = 0; !by_node && si < m->num_stages; si++)
             for (int k = 0; k < m->stages[si].num_out; k++) producer[m->stages[si].out_bufs[k]] = si;
         for (auto &hc : host_out) {
             if (producer[hc.buf] < 0) {
                 overlap = false;
                 break;
             }
-            oc.by_stage[producer[hc.buf]].push_back({hc.host, ptrs[hc.buf], hc.bytes});
+            oc.by_step[producer[hc.buf]].push_back({hc.host, ptrs[hc.buf], hc.bytes});
         }
     }
     if (overlap) {

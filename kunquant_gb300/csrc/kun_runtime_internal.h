@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -50,6 +51,17 @@ struct Arena {
     }
 };
 
+// One kernel of a plan that orders kernels (a stage without a kernel table is
+// one node): what it must follow on other streams, and its own stream.
+struct PlanNode {
+    int stage;
+    int kernel;              // of the stage, or -1: all of it
+    int stream;
+    bool signal;             // a node of another stream follows it
+    std::vector<int> waits;  // nodes of other streams it follows
+    std::vector<int> outs;   // module outputs it writes
+};
+
 // Static execution plan of one module for a (num_stocks, length) shape.
 struct Plan {
     std::vector<int> order;                 // stage ids in a topological order
@@ -57,6 +69,7 @@ struct Plan {
     std::vector<int> temp_slot;             // per buffer: arena slot or -1
     std::vector<std::vector<int>> scratch;  // per stage: slots of its scratch
     std::vector<int> stream_of;             // per stage: stream index
+    std::vector<PlanNode> nodes;            // in launch order; empty: stage by stage
     int num_streams = 1;
     int num_slots = 0;
     size_t slot_bytes = 0;
@@ -70,6 +83,13 @@ uint64_t library_epoch();
 // Builds the stage order and the slot assignment of temporaries and scratch
 // for `nstreams` streams; false (with the error set) on a cyclic stage graph.
 bool make_plan(const KunGpuModuleDesc *m, long long S, long long length, int nstreams, Plan &p);
+
+// Replaces a plan's order and slots by ones in kernels (see kun_plan.cu):
+// `cells` and `rows` (the longest job's) weigh the kernels.  False, leaving
+// the plan as it was, when the stages' kernel tables do not allow it or the
+// slots would exceed `max_slots`.
+bool make_node_plan(const KunGpuModuleDesc *m, double cells, double rows, int nstreams, int max_slots, Plan &p);
+int node_slots(const Plan &p);  // slots it may take where the plan in stages takes p.num_slots
 
 // A captured CUDA graph of one run, valid for the exact buffers it was
 // captured with.
@@ -124,6 +144,11 @@ struct Executor {
     // they were made (call with `mu` held)
     void check_epoch();
 };
+
+// Launches a plan's nodes on the executor's streams, forked from and joined to
+// `origin` (its stream 0): launch(place, node, stream), until it returns false.
+void run_nodes(Executor *ex, const Plan &plan, cudaStream_t origin,
+               const std::function<bool(int, const PlanNode &, cudaStream_t)> &launch);
 
 // Device state of a stream module for `cap` stock columns: per buffer a ring
 // of `window` rows ([window][cap], row n % window holds tick n) and per stage

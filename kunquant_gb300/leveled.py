@@ -527,7 +527,9 @@ class LeveledGen(StageGen):
         plan, ops, lv = self.plan, self.ops, self.plan.lv
         ks = []
         prev_cscans: List[dict] = []
+        made: Dict[int, int] = {}
         for L in plan.levels:
+            done = len(ks)
             if L % 2 == 0:
                 roots = [i for i in range(len(ops)) if plan.is_anchor(i) and lv[i] == L
                          and ops[i]["k"] not in SEQ]
@@ -535,7 +537,7 @@ class LeveledGen(StageGen):
                     roots = self._fuse_into_scans(roots, L, prev_cscans)
                 prev_cscans = []
                 if roots:
-                    for role in self._par_roles(roots, L):
+                    for role in self._par_roles(roots, L, made):
                         ks.append(dict(role, level=L, kind="par"))
             else:
                 roles = []
@@ -560,8 +562,15 @@ class LeveledGen(StageGen):
                         else:
                             whole.append(r)
                     roles = whole
-                if roles:
-                    ks.append({"level": L, "kind": "scan", "roles": roles})
+                by_source: Dict[frozenset, list] = {}
+                for r in roles:
+                    by_source.setdefault(self._sources(r["vr"] | r["wr"], made), []).append(r)
+                for part in by_source.values():
+                    ks.append({"level": L, "kind": "scan", "roles": part})
+            for k in range(done, len(ks)):
+                for r in ks[k].get("roles", [ks[k]]):
+                    for j in r["comp"]:
+                        made[j] = k
         return ks
 
     def _fuse_into_scans(self, roots: List[int], L: int, scans: List[dict]) -> List[int]:
@@ -668,10 +677,24 @@ class LeveledGen(StageGen):
                 w += ops[i]["window"] * 12
         return w
 
-    def _par_roles(self, roots: List[int], L: int) -> List[dict]:
+    def _sources(self, series: Set[int], made: Dict[int, int]) -> frozenset:
+        """What a kernel that reads these series waits for: earlier kernels of
+        the stage, and buffers of other stages."""
+        out = set()
+        for j in series:
+            op = self.ops[j]
+            if op["k"] == "Input":
+                if not self.is_user_input(op):
+                    out.add(("buf", op["buf"]))
+            else:
+                out.add(("kernel", made[j]))
+        return frozenset(out)
+
+    def _par_roles(self, roots: List[int], L: int, made: Dict[int, int]) -> List[dict]:
         """Independent parts of a parallel level (no shared computed op) run as
         separate kernels: each gets its own registers and time chunking.  Cheap
-        pointwise parts are kept together."""
+        pointwise parts with the same sources (_sources) are kept together;
+        `made` maps each earlier kernel's ops to it."""
         plan = self.plan
         closures = []
         for r in roots:
@@ -694,7 +717,12 @@ class LeveledGen(StageGen):
         for g in groups:
             comp = set().union(*[x[1] for x in g])
             (heavy if self._weight(comp) >= 40 else light).append(g)
-        parts = heavy + ([sum(light, [])] if light else [])
+        # cheap parts share a kernel when they wait for the same kernels: one
+        # launch for all would make each wait for all that any of them reads
+        by_source: Dict[frozenset, list] = {}
+        for g in light:
+            by_source.setdefault(self._sources(set().union(*[x[2] | x[3] for x in g]), made), []).extend(g)
+        parts = heavy + list(by_source.values())
         out = []
         for g in parts:
             rts = sorted(sum([x[0] for x in g], []))
@@ -1539,6 +1567,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
             self.scratch[j] = len(self.scratch)
         srcs, calls, kinfo = [], [], []
         tma_src: List[str] = []
+        capped: Set[int] = set()  # kernels with a 64-register instance
         knames = []
         pstruct = f"P_{self.kname}"
         for ki, kd in enumerate(ks):
@@ -1670,11 +1699,14 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
 {chr(10).join(self.lines)}
 }}
 """)
-            # time-parallel kernels also come compiled for 64 registers a
-            # thread (8 blocks of 128 threads an SM), picked per kernel by the
-            # tuner; scan kernels keep one instance
-            for suf, minb in ([("", "KUN_TS_MINB"), ("_r", "8")] if kd["kind"] in ("par", "cscan")
-                              else [("", "KUN_TS_MINB")]):
+            # kernels with window loops or window states also come compiled for
+            # 64 registers a thread (8 blocks of 128 threads an SM), picked per
+            # kernel by the tuner; elementwise kernels need fewer anyway, and
+            # scan kernels keep one instance
+            if kd["kind"] == "cscan" or (kd["kind"] == "par" and any(
+                    ops[i]["k"] in ("ForeachBackWindow", "SkipListState") for i in kd["comp"])):
+                capped.add(ki)
+            for suf, minb in ([("", "KUN_TS_MINB"), ("_r", "8")] if ki in capped else [("", "KUN_TS_MINB")]):
                 srcs.append(f"""__global__ void __launch_bounds__(KUN_TS_THREADS, {minb}) {kname}{suf}(const {pstruct} P) {{
   const int bx = blockIdx.x, by = blockIdx.y;
 {pick}
@@ -1701,6 +1733,8 @@ struct {pstruct} {{
 }};
 """
         self.kernel_info = [(d << 1) | sc for d, sc in kinfo]
+        for kd in ks:
+            self.kernel_info += self._kernel_io(kd)
         self.num_kernels_override = nk
         # per kernel: time tile (or roles) and block size, from the tuning
         # arrays when given
@@ -1715,25 +1749,55 @@ struct {pstruct} {{
         for k, (d, sc) in enumerate(kinfo):
             gy = str(d) if sc else f"(unsigned)((a->length + P.tile[{k}] - 1) / P.tile[{k}])"
             grid = f"dim3((unsigned)((a->num_stocks + blk{k} - 1) / blk{k}), {gy}), blk{k}, 0, (cudaStream_t)stream"
-            if sc:
-                calls.append(f"  {knames[k]}<<<{grid}>>>(P);")
-            elif k in self.tma_kernels:
+            calls.append(f"  if (a->only_kernel == 0 || a->only_kernel == {k + 1}) {{")
+            if k in self.tma_kernels:
                 # the staged instance: 128 threads, rows of whole 16-byte
                 # units (S % 4 == 0) from 16-byte aligned series
                 ok = " && ".join([f"kun::aligned16({e})" for e in self.tma_kernels[k]])
                 calls.append(f"  if (kun::tma_enabled() && blk{k} == 128 && (a->num_stocks % 4) == 0 && {ok}) "
                              f"{knames[k]}_tma<<<{grid}>>>(P);\n"
-                             f"  else if (tb{k} & KUN_BLOCK_REGCAP) {knames[k]}_r<<<{grid}>>>(P);\n"
                              f"  else {knames[k]}<<<{grid}>>>(P);")
-            else:
+            elif k in capped:
                 calls.append(f"  if (tb{k} & KUN_BLOCK_REGCAP) {knames[k]}_r<<<{grid}>>>(P);\n"
                              f"  else {knames[k]}<<<{grid}>>>(P);")
-            calls.append("  if (cudaError_t e = cudaGetLastError()) return (int)e;")
+            else:
+                calls.append(f"  {knames[k]}<<<{grid}>>>(P);")
+            calls.append("  if (cudaError_t e = cudaGetLastError()) return (int)e;\n  }")
         launch = self.launcher(pstruct, "\n".join(sel + calls))
-        launch += self._group_launcher(pstruct, knames, kinfo)
+        launch += self._group_launcher(pstruct, knames, kinfo, capped)
         return head + "".join(srcs) + "".join(tma_src), launch
 
-    def _group_launcher(self, pstruct: str, knames: List[str], kinfo) -> str:
+    def _kernel_io(self, kd: dict) -> List[int]:
+        """[instructions a cell, reads, ..., writes, ...] of a kernel for the
+        module table: the runtime orders kernels by what they read and write."""
+        ops = self.ops
+        reads, writes, cost = set(), set(), 0.0
+        for r in kd.get("roles", [kd]):
+            comp = r["comp"]
+            for j in r["vr"] | r["wr"]:
+                if ops[j]["k"] != "Input":
+                    reads.add(-1 - self.scratch[j] if j in self.scratch else ops[j]["buf"])
+                elif not (self.is_user_input(ops[j]) or ops[j].get("single_value")):
+                    reads.add(ops[j]["buf"])
+            # a scan stores its roots, a time-parallel kernel whatever it computes
+            stored = comp if kd["kind"] == "par" else set(r["roots"])
+            made = ({j for j in comp if ops[j]["k"] in ("Output", "WindowedTempOutput")}
+                    | {j for j in stored if j in self.scratch})
+            for j in made:
+                writes.add(ops[j]["buf"] if ops[j]["k"] == "Output" else -1 - self.scratch[j])
+            cost += 15 * (len(r["vr"] | r["wr"]) + len(made)) + 4 * len(comp)
+            for i in comp:
+                if ops[i]["k"] == "ForeachBackWindow":
+                    inner = sum(1 for j in comp if ops[j].get("p", -1) == i)
+                    reds = sum(1 for j in comp if ops[j]["k"] in REDUCTIONS
+                               and contraction.reduction_loop(ops, j) in self.plan.loop_chain[i])
+                    cost += (ops[i]["window"] - ops[i].get("segment_end", 0)) * (inner + 5 * reds)
+                elif ops[i]["k"] == "SkipListState":
+                    cost += 10 * ops[i]["window"]
+        reads -= writes
+        return [int(cost), len(reads)] + sorted(reads) + [len(writes)] + sorted(writes)
+
+    def _group_launcher(self, pstruct: str, knames: List[str], kinfo, capped: Set[int]) -> str:
         """prepare(): the parameter blocks of n jobs; launch_group(): every
         kernel of the stage once over all jobs' tiles."""
         fill = "\n".join(f"    P.p[{sl}] = a->buffers[{bid}];" for bid, sl in self.slots.items())
@@ -1749,11 +1813,11 @@ struct {pstruct} {{
             gy = str(d) if sc else f"(a->length + tile - 1) / tile"
             tl = "0" if sc else f"(a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : {d}"
             kcall = (f"{knames[k]}_grp<<<(unsigned)total, blk, 0, (cudaStream_t)stream>>>((const {pstruct}*)dev, tt);"
-                     if sc else
+                     if k not in capped else
                      f"if (tb & KUN_BLOCK_REGCAP) {knames[k]}_r_grp<<<(unsigned)total, blk, 0, (cudaStream_t)stream>>>"
                      f"((const {pstruct}*)dev, tt);\n      else {knames[k]}_grp<<<(unsigned)total, blk, 0, "
                      f"(cudaStream_t)stream>>>((const {pstruct}*)dev, tt);")
-            launches.append(f"""  {{
+            launches.append(f"""  if (args[0].only_kernel == 0 || args[0].only_kernel == {k + 1}) {{
     const int tb = (args[0].tune_block && args[0].tune_block[{k}] > 0) ? args[0].tune_block[{k}] : KUN_TS_THREADS;
     const int blk = tb & 0xffff;
     kun::TileTable tt;
