@@ -641,17 +641,6 @@ inline int launch_ts_to_sts(const T *in, T *out, long long S, long long length, 
     return (int)cudaGetLastError();
 }
 
-inline int kun_num_sms() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 132;
-    }
-    return n;
-}
-
 template <typename Kernel> inline int rank_smem_limit(Kernel kernel, size_t smem) {
     if (smem <= kSmemOptIn) return 0;
     return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -1568,6 +1568,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
         srcs, calls, kinfo = [], [], []
         tma_src: List[str] = []
         capped: Set[int] = set()  # kernels with a 64-register instance
+        warm: Dict[int, int] = {}  # rows a tile runs before its own
         knames = []
         pstruct = f"P_{self.kname}"
         for ki, kd in enumerate(ks):
@@ -1622,6 +1623,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
                     self.vec_u = U
                 self.lines.append("  }")
                 kinfo.append((chunk, 0))
+                warm[ki] = wmax
                 if not (sls or wide) and U == VEC_U_ELEM and self._tma_eligible(comp, vr, wr):
                     tma_src.append(self._tma_kernel(kname, pstruct, ki, comp, vr, stores, loops, decl, U))
             elif kd["kind"] == "cscan":
@@ -1646,6 +1648,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
                 self.lines += self._moment_decls("  ")
                 self._scan_prefetch(r, self._scan_block(r), "  ", chunk=True)
                 kinfo.append((max(64, (2 * wmax + 15) // 16 * 16), 0))
+                warm[ki] = wmax
             else:
                 roles = kd["roles"]
                 self.lines.append("  switch (by) {")
@@ -1743,7 +1746,8 @@ struct {pstruct} {{
             sel.append(f"  const int tb{k} = (a->tune_block && a->tune_block[{k}] > 0) ? a->tune_block[{k}] : KUN_TS_THREADS;")
             sel.append(f"  const int blk{k} = tb{k} & 0xffff;")
             if not sc:
-                sel.append(f"  P.tile[{k}] = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : {d};")
+                sel.append(f"  P.tile[{k}] = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : "
+                           f"kun::pick_tile(a, 1, {d}, {warm[k]}, blk{k});")
             else:
                 sel.append(f"  P.tile[{k}] = 0;")
         for k, (d, sc) in enumerate(kinfo):
@@ -1764,7 +1768,7 @@ struct {pstruct} {{
                 calls.append(f"  {knames[k]}<<<{grid}>>>(P);")
             calls.append("  if (cudaError_t e = cudaGetLastError()) return (int)e;\n  }")
         launch = self.launcher(pstruct, "\n".join(sel + calls))
-        launch += self._group_launcher(pstruct, knames, kinfo, capped)
+        launch += self._group_launcher(pstruct, knames, kinfo, capped, warm)
         return head + "".join(srcs) + "".join(tma_src), launch
 
     def _kernel_io(self, kd: dict) -> List[int]:
@@ -1797,21 +1801,28 @@ struct {pstruct} {{
         reads -= writes
         return [int(cost), len(reads)] + sorted(reads) + [len(writes)] + sorted(writes)
 
-    def _group_launcher(self, pstruct: str, knames: List[str], kinfo, capped: Set[int]) -> str:
+    def _group_launcher(self, pstruct: str, knames: List[str], kinfo, capped: Set[int],
+                        warm: Dict[int, int]) -> str:
         """prepare(): the parameter blocks of n jobs; launch_group(): every
         kernel of the stage once over all jobs' tiles."""
         fill = "\n".join(f"    P.p[{sl}] = a->buffers[{bid}];" for bid, sl in self.slots.items())
         fillw = "\n".join(f"    P.w[{sc}] = a->scratch[{sc}];" for sc in range(len(self.scratch)))
-        tiles = []
+        tiles, picks = [], []
         for k, (d, sc) in enumerate(kinfo):
             if sc:
                 tiles.append(f"    P.tile[{k}] = 0;")
-            else:
-                tiles.append(f"    P.tile[{k}] = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : {d};")
+                continue
+            # one tile for the group, from all its jobs' rows
+            picks.append(f"  int tile{k};\n  {{\n    const KunGpuStageArgs* a = &args[0];\n"
+                         f"    const int tb = (a->tune_block && a->tune_block[{k}] > 0) ? a->tune_block[{k}] : KUN_TS_THREADS;\n"
+                         f"    tile{k} = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : "
+                         f"kun::pick_tile(args, njobs, {d}, {warm[k]}, tb & 0xffff);\n  }}")
+            tiles.append(f"    P.tile[{k}] = tile{k};")
         launches = []
         for k, (d, sc) in enumerate(kinfo):
             gy = str(d) if sc else f"(a->length + tile - 1) / tile"
-            tl = "0" if sc else f"(a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : {d}"
+            tl = ("0" if sc else f"(args[0].tune_tile && args[0].tune_tile[{k}] > 0) ? args[0].tune_tile[{k}] : "
+                  f"kun::pick_tile(args, njobs, {d}, {warm[k]}, blk)")
             kcall = (f"{knames[k]}_grp<<<(unsigned)total, blk, 0, (cudaStream_t)stream>>>((const {pstruct}*)dev, tt);"
                      if k not in capped else
                      f"if (tb & KUN_BLOCK_REGCAP) {knames[k]}_r_grp<<<(unsigned)total, blk, 0, (cudaStream_t)stream>>>"
@@ -1822,11 +1833,11 @@ struct {pstruct} {{
     const int blk = tb & 0xffff;
     kun::TileTable tt;
     tt.njobs = njobs;
+    const long long tile = {tl};
+    (void)tile;
     long long total = 0;
     for (int j = 0; j < njobs; ++j) {{
       const KunGpuStageArgs* a = &args[j];
-      const long long tile = {tl};
-      (void)tile;
       tt.off[j] = (int)total;
       if (a->num_stocks > 0 && a->length > 0) total += ((a->num_stocks + blk - 1) / blk) * (long long)({gy});
     }}
@@ -1839,7 +1850,8 @@ struct {pstruct} {{
   }}""")
         return f"""
 extern "C" size_t {self.kname}_prepare(const KunGpuStageArgs* args, int njobs, void* host) {{
-  if (host) {{
+  if (host && njobs > 0) {{
+{chr(10).join(picks)}
     for (int j = 0; j < njobs; ++j) {{
       const KunGpuStageArgs* a = &args[j];
       {pstruct}& P = (({pstruct}*)host)[j];
