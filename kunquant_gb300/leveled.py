@@ -1746,8 +1746,9 @@ struct {pstruct} {{
             sel.append(f"  const int tb{k} = (a->tune_block && a->tune_block[{k}] > 0) ? a->tune_block[{k}] : KUN_TS_THREADS;")
             sel.append(f"  const int blk{k} = tb{k} & 0xffff;")
             if not sc:
-                sel.append(f"  P.tile[{k}] = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : "
-                           f"kun::pick_tile(a, 1, {d}, {warm[k]}, blk{k});")
+                tuned = f"(a->tune_tile && a->tune_tile[{k}] > 0)"
+                sel.append(f"  P.tile[{k}] = {tuned} ? a->tune_tile[{k}] : {d};")
+                sel.append(f"  if (!{tuned}) P.tile[{k}] = kun::pick_tile(a, 1, P.tile[{k}], {warm[k]}, blk{k});")
             else:
                 sel.append(f"  P.tile[{k}] = 0;")
         for k, (d, sc) in enumerate(kinfo):
