@@ -1474,6 +1474,8 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
         src = {r: ops[ops[r]["in"][0]]["in"][1] for r in reds}
         kind = {r: self.EXT_KINDS[ops[r]["k"]] for r in reds}
 
+        pos = "float" if T == "float" else "int"  # kun::RExt::P
+
         def ext(r):
             mx, arg = kind[r]
             return f"kun::RExt<{T}, {mx}, {arg}>"
@@ -1495,7 +1497,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
             for s in sorted({src[r] for r in active}):
                 L.append(f"{bi}  const {T} x{s} = {self._vload(s, 't - d')};")
             for r in active:
-                L.append(f"{bi}  c{r}.step(x{src[r]}, ({T})(-d));")
+                L.append(f"{bi}  c{r}.step(x{src[r]}, ({pos})(-d));")
             L.append(f"{bi}}}")
         # the edge rows: o{s}_{w}[k] = row t+1-w+k, n{s}[k] = row t+1+k (k < U-1)
         for s, w in sorted({(src[r], win[r]) for r in reds}):
@@ -1514,11 +1516,11 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
             L.append(f"{bj}{{")
             L.append(f"{bj}  {ext(r)} a;")
             L.append(f"{bj}  #pragma unroll")
-            L.append(f"{bj}  for (int k = u; k < {U - 1}; ++k) a.step(o{s}_{w}[k], ({T})(k + 1 - {w}));")
+            L.append(f"{bj}  for (int k = u; k < {U - 1}; ++k) a.step(o{s}_{w}[k], ({pos})(k + 1 - {w}));")
             L.append(f"{bj}  a.then(c{r});")
             L.append(f"{bj}  #pragma unroll")
-            L.append(f"{bj}  for (int k = 0; k < u; ++k) a.step(n{s}[k], ({T})(k + 1));")
-            res = f"a.arg(({T})u)" if kind[r][1] == "true" else "a.v"
+            L.append(f"{bj}  for (int k = 0; k < u; ++k) a.step(n{s}[k], ({pos})(k + 1));")
+            res = f"a.arg(({pos})u)" if kind[r][1] == "true" else "a.v"
             L.append(f"{bj}  r{r}[u].v = {res};")
             L.append(f"{bj}}}")
         L.append(f"{bi}}}")

@@ -115,7 +115,8 @@ class StreamGen(StageGen):
         if k == "SkipListState":
             W = op["window"]
             if W <= 64:
-                return f"kun::RegWindow<{T}, {W}, {'true' if self._sl_idx(i) else 'false'}> sl{i};"
+                # its values are the state's arrays: kept as values
+                return f"kun::RegWindow<{T}, {W}, {'true' if self._sl_idx(i) else 'false'}, kun::AsValue<{T}>> sl{i};"
             return f"kun::SortedWindow<{W}> sl{i};"
         if k == "Accumulator":
             return f"{T} acc{i} = 0;"
