@@ -689,9 +689,11 @@ template <> struct LogTables<{T}> {{
     for si in extern_init:
         lines.append(f'extern "C" int kst_{tag}_{si}_init(const KunGpuStageArgs*, void*);')
     for si, ki in kinfo.items():
+        lines.append(f"static const int32_t st{si}_kinfo[] = {{{', '.join(str(v) for v in ki)}}};")
+        if spec["output_layout"] == "STREAM":
+            continue
         lines.append(f'extern "C" size_t kst_{tag}_{si}_prepare(const KunGpuStageArgs*, int, void*);')
         lines.append(f'extern "C" int kst_{tag}_{si}_launch_group(const KunGpuStageArgs*, int, const void*, void*);')
-        lines.append(f"static const int32_t st{si}_kinfo[] = {{{', '.join(str(v) for v in ki)}}};")
     for si, mx in imax.items():
         lines.append(f"static const int32_t st{si}_imax[] = {{{', '.join(str(v) for v in mx)}}};")
     for si, st in enumerate(spec["stages"]):
@@ -708,8 +710,9 @@ template <> struct LogTables<{T}> {{
                      f"{st.get('pending', 0)}, {scratch_counts[si]}, 0, kst_{tag}_{si}_launch, {kernel_counts[si]}, "
                      f"{state_t[si]}, {state_i[si]}, {init_fn[si]}, "
                      + (f"st{si}_imax, " if si in imax else "nullptr, ")
-                     + (f"st{si}_kinfo, kst_{tag}_{si}_prepare, kst_{tag}_{si}_launch_group}},"
-                        if si in kinfo else "nullptr, nullptr, nullptr},"))
+                     + (f"st{si}_kinfo, " if si in kinfo else "nullptr, ")
+                     + (f"kst_{tag}_{si}_prepare, kst_{tag}_{si}_launch_group}},"
+                        if si in kinfo and spec["output_layout"] != "STREAM" else "nullptr, nullptr},"))
     lines.append("};")
     bk = {"INPUT": "KUN_BUF_INPUT", "OUTPUT": "KUN_BUF_OUTPUT", "TEMP": "KUN_BUF_TEMP"}
     lines.append(f"static const KunGpuBufferDesc buffers_{tag}[] = {{")

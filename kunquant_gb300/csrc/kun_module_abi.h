@@ -109,7 +109,9 @@ typedef struct {
      * these num_kernels entries, per kernel: the instructions a cell takes
      * (an estimate), the number of series it reads from other kernels and
      * those, the number it writes and those; a series is a buffer id, or
-     * -1 - k for the stage's scratch k */
+     * -1 - k for the stage's scratch k.  Time-series stages of a stream
+     * module: the same table of their launch units (entries and instructions
+     * 0) */
     const int32_t *kernel_info;
     KunGpuPrepareFn prepare;
     KunGpuGroupLaunchFn launch_group;

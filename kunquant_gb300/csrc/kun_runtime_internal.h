@@ -182,16 +182,21 @@ struct TickSchedule {
 bool make_tick_schedule(const KunGpuModuleDesc *m, const std::vector<int> &order, int nstreams, TickSchedule &s);
 void free_tick_schedule(TickSchedule &s);
 
-// A tick as a chain of stage-graph levels: level d holds the stages whose
-// longest path from a source has d stages, so the stages of a level do not
-// depend on each other.  The Rank stages of a level run as one launch over
-// (segment, stage) blocks; every other stage keeps its own launch.  All on
-// one stream: a tick is a short chain of launches instead of one launch per
-// stage with cross-stream events.
+// A tick as a chain of levels: level d holds the launch units (of time-series
+// stages) and the cross-sectional stages whose longest path from a source has
+// d of them, so those of a level do not depend on each other.  The Rank
+// stages of a level run as one launch over (segment, stage) blocks; the units
+// run beside it on `side`, forked from and joined to the tick's stream.
 struct TickLevels {
-    std::vector<std::vector<int>> other;  // per level: non-Rank stages
-    std::vector<int> rank_off, rank_cnt;  // per level: slice of the job table
-    void *d_jobs = nullptr;               // device RankJob table
+    struct Unit {
+        int stage, kernel;  // kernel -1: the whole stage
+    };
+    std::vector<std::vector<Unit>> other;  // per level: all but the Rank stages
+    std::vector<int> rank_off, rank_cnt;   // per level: slice of the job table
+    void *d_jobs = nullptr;                // device RankJob table
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> join;
+    cudaEvent_t fork = nullptr;
     bool ok = false;
 };
 // false when a Rank stage does not read and write exactly one ring

@@ -180,28 +180,40 @@ void free_tick_schedule(TickSchedule &s) {
 // Enqueue one tick of every stage for the segments in d_seg / d_tick: in
 // order on `st`, or with `sched`, on its streams (forked from and joined back
 // into `st`) with events for the cross-stream dependencies.
+static constexpr int kSideStreams = 7;  // launches of a level beside the tick's stream
+
 bool make_tick_levels(const StreamStore &store, const std::vector<int> &order, TickLevels &lv) {
     const KunGpuModuleDesc *m = store.m;
-    const int ns = m->num_stages;
-    std::vector<int> depth(ns, 0);
-    for (int si : order)  // a topological order: predecessors come first
-        for (int d = 0; d < m->stages[si].num_deps; d++) {
-            const int j = m->stages[si].deps[d];
-            if (j >= 0) depth[j] = std::max(depth[j], depth[si] + 1);
+    // depth of every unit from the depths of the values it reads
+    std::vector<int> made(m->num_buffers, -1);  // level that writes the buffer
+    std::vector<std::vector<int>> ranks;
+    auto place = [&](int stage, int kernel, const int32_t *reads, int nr, const int32_t *writes, int nw) {
+        int d = 0;
+        for (int k = 0; k < nr; k++) d = std::max(d, made[reads[k]] + 1);
+        for (int k = 0; k < nw; k++) made[writes[k]] = d;
+        if (d >= (int)lv.other.size()) {
+            lv.other.resize(d + 1);
+            ranks.resize(d + 1);
         }
-    int nl = 0;
-    for (int si : order) nl = std::max(nl, depth[si] + 1);
-    std::vector<std::vector<int>> ranks(nl);
-    lv.other.assign(nl, {});
-    for (int si : order) {
+        if (m->stages[stage].kind == KUN_STAGE_RANK) ranks[d].push_back(stage);
+        else lv.other[d].push_back({stage, kernel});
+    };
+    lv.other.clear();
+    for (int si : order) {  // a topological order: predecessors come first
         const KunGpuStageDesc &d = m->stages[si];
-        if (d.kind == KUN_STAGE_RANK) {
-            if (d.num_in != 1 || d.num_out != 1) return false;
-            ranks[depth[si]].push_back(si);
-        } else {
-            lv.other[depth[si]].push_back(si);
+        if (d.kind == KUN_STAGE_RANK && (d.num_in != 1 || d.num_out != 1)) return false;
+        if (!d.kernel_info) {
+            place(si, -1, d.in_bufs, d.num_in, d.out_bufs, d.num_out);
+            continue;
+        }
+        const int32_t *q = d.kernel_info + d.num_kernels;
+        for (int k = 0; k < d.num_kernels; k++) {
+            const int nr = q[1], nw = q[2 + nr];
+            place(si, k, q + 2, nr, q + 3 + nr, nw);
+            q += 3 + nr + nw;
         }
     }
+    const int nl = (int)lv.other.size();
     std::vector<kun::RankJob> jobs;
     lv.rank_off.assign(nl, 0);
     lv.rank_cnt.assign(nl, 0);
@@ -227,17 +239,32 @@ bool make_tick_levels(const StreamStore &store, const std::vector<int> &order, T
             cudaSuccess)
             return false;
     }
+    lv.side.assign(kSideStreams, nullptr);
+    lv.join.assign(kSideStreams, nullptr);
+    for (int k = 0; k < kSideStreams; k++)
+        if (cudaStreamCreateWithFlags(&lv.side[k], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&lv.join[k], cudaEventDisableTiming) != cudaSuccess)
+            return false;
+    if (cudaEventCreateWithFlags(&lv.fork, cudaEventDisableTiming) != cudaSuccess) return false;
     lv.ok = true;
     return true;
 }
 
 void free_tick_levels(TickLevels &lv) {
     if (lv.d_jobs) cudaFree(lv.d_jobs);
+    for (auto q : lv.side)
+        if (q) cudaStreamDestroy(q);
+    for (auto e : lv.join)
+        if (e) cudaEventDestroy(e);
+    if (lv.fork) cudaEventDestroy(lv.fork);
+    lv.side.clear();
+    lv.join.clear();
+    lv.fork = nullptr;
     lv.d_jobs = nullptr;
     lv.ok = false;
 }
 
-static KunStatus launch_stage(const StreamStore &store, int si, const int32_t *d_seg_off, const int32_t *d_seg_stock0,
+static KunStatus launch_stage(const StreamStore &store, int si, int kernel, const int32_t *d_seg_off, const int32_t *d_seg_stock0,
                               const int64_t *d_tick, int nseg, long long n_active, int max_len, cudaStream_t sst,
                               const int32_t *d_seg_count) {
     const KunGpuStageDesc &d = store.m->stages[si];
@@ -256,6 +283,7 @@ static KunStatus launch_stage(const StreamStore &store, int si, const int32_t *d
     a.n_active = n_active;
     a.max_seg_len = max_len;
     a.seg_count = d_seg_count;
+    a.only_kernel = kernel + 1;
     int rc = d.launch(&a, (void *)sst);
     if (rc) {
         set_error("stage %d (%s) failed: %s", si, d.name, cudaGetErrorString((cudaError_t)rc));
@@ -271,9 +299,16 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
     const KunGpuModuleDesc *m = store.m;
     if (levels && levels->ok) {
         for (size_t l = 0; l < levels->other.size(); l++) {
-            for (int si : levels->other[l]) {
-                KunStatus rs = launch_stage(store, si, d_seg_off, d_seg_stock0, d_tick, nseg, n_active, max_len, st,
-                                            d_seg_count);
+            // the level's first launch stays on the tick's stream
+            const auto &units = levels->other[l];
+            const size_t here = levels->rank_cnt[l] > 0 ? 0 : 1;
+            const size_t sides = std::min(units.size() > here ? units.size() - here : 0, levels->side.size());
+            if (sides) cudaEventRecord(levels->fork, st);
+            for (size_t k = 0; k < sides; k++) cudaStreamWaitEvent(levels->side[k], levels->fork, 0);
+            for (size_t u = 0; u < units.size(); u++) {
+                cudaStream_t on = u < here || !sides ? st : levels->side[(u - here) % sides];
+                KunStatus rs = launch_stage(store, units[u].stage, units[u].kernel, d_seg_off, d_seg_stock0, d_tick,
+                                            nseg, n_active, max_len, on, d_seg_count);
                 if (rs != KUN_SUCCESS) return rs;
             }
             if (levels->rank_cnt[l] > 0) {
@@ -290,6 +325,10 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
                     set_error("rank stages of level %d failed: %s", (int)l, cudaGetErrorString((cudaError_t)rc));
                     return KUN_CUDA_ERROR;
                 }
+            }
+            for (size_t k = 0; k < sides; k++) {
+                cudaEventRecord(levels->join[k], levels->side[k]);
+                cudaStreamWaitEvent(st, levels->join[k], 0);
             }
         }
         return KUN_SUCCESS;

@@ -7,6 +7,7 @@
 //    stock order (sequential, as the reference adds), then x / sum.
 //  - DiffWithWeightedSum (KunQuant/ops/MiscOp.py:220-240).
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "kun_device.cuh"
@@ -641,6 +642,8 @@ inline int launch_ts_to_sts(const T *in, T *out, long long S, long long length, 
     return (int)cudaGetLastError();
 }
 
+constexpr long long kGridRows = 1ll << 30;  // rows of one launch
+
 template <typename Kernel> inline int rank_smem_limit(Kernel kernel, size_t smem) {
     if (smem <= kSmemOptIn) return 0;
     return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -676,7 +679,9 @@ inline int launch_rank(const T *in, T *out, long long S, long long length, cudaS
         const int nt = rank_threads((int)S, I);
         const size_t smem = rank_smem_bytes<T>(nt, I);
         if (int e = rank_smem_limit(rank_rows<T, I, M>, smem)) return e;
-        rank_rows<T, I, M><<<(unsigned)length, nt, smem, st>>>(in, out, (int)S);
+        for (long long t = 0; t < length; t += kGridRows)
+            rank_rows<T, I, M>
+                <<<(unsigned)std::min(length - t, kGridRows), nt, smem, st>>>(in + t * S, out + t * S, (int)S);
         return (int)cudaGetLastError();
     });
 }
@@ -693,9 +698,10 @@ struct RankRowsJob {
 // A block has the threads of the longest row; a shorter row's surplus warps
 // leave at once and its barriers count only the others.
 template <typename T, int ITEMS, int MAXT>
-__global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_rows_multi(const RankRowsJob *__restrict__ jobs, int njobs) {
+__global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT))
+    rank_rows_multi(const RankRowsJob *__restrict__ jobs, int njobs, long long first_row) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const long long r = blockIdx.x;
+    const long long r = first_row + blockIdx.x;
     int lo = 0, hi = njobs - 1;  // the job whose rows hold r
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -716,13 +722,14 @@ template <typename T>
 inline int launch_rank_rows_multi(const RankRowsJob *d_jobs, int njobs, long long total_rows, long long max_S,
                                   cudaStream_t st) {
     if (njobs <= 0 || total_rows <= 0) return 0;
-    if (total_rows > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
     return rank_dispatch<false>(max_S, [&](auto items, auto maxt) {
         constexpr int I = decltype(items)::value, M = decltype(maxt)::value;
         const int nt = rank_threads((int)max_S, I);
         const size_t smem = rank_smem_bytes<T>(nt, I);
         if (int e = rank_smem_limit(rank_rows_multi<T, I, M>, smem)) return e;
-        rank_rows_multi<T, I, M><<<(unsigned)total_rows, nt, smem, st>>>(d_jobs, njobs);
+        for (long long r = 0; r < total_rows; r += kGridRows)
+            rank_rows_multi<T, I, M>
+                <<<(unsigned)std::min(total_rows - r, kGridRows), nt, smem, st>>>(d_jobs, njobs, r);
         return (int)cudaGetLastError();
     });
 }

@@ -35,8 +35,80 @@ __device__ __forceinline__ int kun_segment(const int32_t* __restrict__ off, int 
 """
 
 
+def stage_parts(ops: List[dict]) -> List[List[int]]:
+    """The ops of a time-series stage in parts that share no computed value
+    (inputs and constants aside), each in op order."""
+    n = len(ops)
+    parent = list(range(n))
+
+    def find(x):
+        while parent[x] != x:
+            parent[x] = parent[parent[x]]
+            x = parent[x]
+        return x
+
+    source = [op["k"] in ("Input", "ConstantOp") for op in ops]
+    prev_loop = None
+    for i, op in enumerate(ops):
+        if source[i]:
+            continue
+        for j in list(op["in"]) + ([op["p"]] if op.get("p", -1) >= 0 else []):
+            if not source[j]:
+                parent[find(i)] = find(j)
+        if op["k"] == "ForeachBackWindow":
+            if op.get("copy_prev_body") and prev_loop is not None:
+                parent[find(i)] = find(prev_loop)
+            prev_loop = i
+    parts: Dict[int, List[int]] = {}
+    for i in range(n):
+        if not source[i]:
+            parts.setdefault(find(i), []).append(i)
+    return sorted(parts.values())
+
+
+_plans: List[tuple] = []
+
+
+def tick_groups(spec: dict) -> Dict[int, List[List[List[int]]]]:
+    """Per time-series stage its parts in groups of equal depth, the depth of a
+    part being the longest chain of parts and cross-sectional stages before
+    it: the parts of one depth, of all stages, do not depend on each other."""
+    for known, groups in _plans:
+        if known is spec:
+            return groups
+    nodes = []  # (stage, part or None, reads, writes)
+    for si, st in enumerate(spec["stages"]):
+        if st["kind"] != "ts":
+            nodes.append((si, None, set(st["in"]), set(st["out"])))
+            continue
+        ops = st["ops"]
+        for part in stage_parts(ops):
+            reads = {ops[j]["buf"] for i in part for j in ops[i]["in"] if ops[j]["k"] == "Input"}
+            nodes.append((si, part, reads, {ops[i]["buf"] for i in part if ops[i]["k"] == "Output"}))
+    writer = {b: k for k, node in enumerate(nodes) for b in node[3]}
+    depth: Dict[int, int] = {}
+
+    def depth_of(k):
+        if k not in depth:
+            depth[k] = max([depth_of(writer[b]) + 1 for b in nodes[k][2] if b in writer and writer[b] != k],
+                           default=0)
+        return depth[k]
+
+    by_stage: Dict[int, Dict[int, list]] = {}
+    for k, (si, part, _, _) in enumerate(nodes):
+        if part is not None:
+            by_stage.setdefault(si, {}).setdefault(depth_of(k), []).append(part)
+    groups = {si: [by_stage[si][d] for d in sorted(by_stage[si])] for si in by_stage}
+    _plans[:] = _plans[-7:] + [(spec, groups)]
+    return groups
+
+
 class StreamGen(StageGen):
-    """Tick kernel, state initialiser and launchers of one stream stage."""
+    """Tick kernels, state initialiser and launchers of one stream stage.
+
+    One thread works on one part (stage_parts) of one stock: a thread that
+    walked all of a stage's windows took up to 100 us of a tick, and the
+    stages' chain 39 levels where the parts' has 10."""
 
     def __init__(self, spec: dict, si: int, tag: str):
         super().__init__(spec, si, tag)
@@ -152,39 +224,56 @@ class StreamGen(StageGen):
             W = int(ops[i].get("window", 0))
             self.state_i_max += [-1 if f.startswith(("ix[", "idx[")) else W for f in inf]
         self.has_init = bool(fields)
-        # rings of the buffers the stage touches
-        decl = []
-        for i, op in enumerate(ops):
-            if op["k"] in ("Input", "Output") or (op["k"] == "WindowedTempOutput" and op.get("p", -1) < 0):
-                if op.get("single_value"):
-                    raise RuntimeError("single-value inputs are not supported in stream mode")
-                sl = self.slot(op["buf"])
-                decl.append(f"  {T}* __restrict__ r{i} = ({T}*)P.p[{sl}] + s;")
-        loads, stores = [], []
-        for i, (tf, inf) in fields.items():
-            loads.append(f"  {self._state_decl(i)}")
-            W = ops[i].get("window", 0)
-            big_sl = ops[i]["k"] == "SkipListState" and W > 64
-            for j, f in enumerate(tf):
-                tgt = self._field(i, f)
-                src = f"st[{toff[i] + j} * S]"
-                loads.append(f"  {tgt} = {'(double)' if big_sl else ''}{src};")
-                stores.append(f"  {src} = ({T}){tgt};")
-            for j, f in enumerate(inf):
-                tgt = self._field(i, f)
-                src = f"si[{ioff[i] + j} * S]"
-                loads.append(f"  {tgt} = {src};")
-                stores.append(f"  {src} = {tgt};")
-        # ops of one tick (CodegenCpp.py:189-307 with length 1)
-        self.lines = []
-        self.ring_ws = set()
+        # ops of one tick (CodegenCpp.py:189-307 with length 1), part by part
+        groups = tick_groups(self.spec)[self.si]
+        parts = [part for group in groups for part in group]
         loops = self._loops()
-        for i, op in enumerate(ops):
-            if op.get("p", -1) >= 0:
-                continue
-            self._emit(i, loops)
-        body = "\n".join(self.lines)
-        ring_pos = "\n".join(f"  const int nm{W} = (int)(n % {W});" for W in sorted(self.ring_ws))
+        cases = []
+        for c, part in enumerate(parts):
+            used = set(part)
+            for i in part:
+                used |= {j for j in ops[i]["in"] if ops[j]["k"] in ("Input", "ConstantOp")}
+            decl, loads, stores = [], [], []
+            for i in sorted(used):
+                op = ops[i]
+                if op["k"] in ("Input", "Output") or (op["k"] == "WindowedTempOutput" and op.get("p", -1) < 0):
+                    if op.get("single_value"):
+                        raise RuntimeError("single-value inputs are not supported in stream mode")
+                    sl = self.slot(op["buf"])
+                    decl.append(f"  {T}* __restrict__ r{i} = ({T}*)P.p[{sl}] + s;")
+            for i in part:
+                if i not in fields:
+                    continue
+                tf, inf = fields[i]
+                loads.append(f"  {self._state_decl(i)}")
+                W = ops[i].get("window", 0)
+                big_sl = ops[i]["k"] == "SkipListState" and W > 64
+                for j, f in enumerate(tf):
+                    tgt = self._field(i, f)
+                    src = f"st[{toff[i] + j} * S]"
+                    loads.append(f"  {tgt} = {'(double)' if big_sl else ''}{src};")
+                    stores.append(f"  {src} = ({T}){tgt};")
+                for j, f in enumerate(inf):
+                    tgt = self._field(i, f)
+                    src = f"si[{ioff[i] + j} * S]"
+                    loads.append(f"  {tgt} = {src};")
+                    stores.append(f"  {src} = {tgt};")
+            self.lines = []
+            self.ring_ws = set()
+            for i in sorted(used):
+                if ops[i].get("p", -1) < 0:
+                    self._emit(i, loops)
+            ring_pos = [f"  const int nm{W} = (int)(n % {W});" for W in sorted(self.ring_ws)]
+            cases.append("\n".join([f"  case {c}: {{"] + ring_pos + decl + loads + self.lines + stores + ["  } break;"]))
+        # launch units: the groups, with what each reads and writes
+        self.num_kernels_override = len(groups)
+        self.kernel_info = [0] * len(groups)
+        for group in groups:
+            reads = sorted({ops[j]["buf"] for part in group for i in part for j in ops[i]["in"]
+                            if ops[j]["k"] == "Input" and self.bufs[ops[j]["buf"]]["kind"] != "INPUT"})
+            writes = sorted({ops[i]["buf"] for part in group for i in part if ops[i]["k"] == "Output"})
+            self.kernel_info += [0, len(reads)] + reads + [len(writes)] + writes
+        first = [sum(len(g) for g in groups[:k]) for k in range(len(groups))]
         pstruct = f"P_{self.kname}"
         nslots = max(1, len(self.slots))
         src = _SEG_HELPER + f"""
@@ -197,6 +286,7 @@ struct {pstruct} {{
   const long long* seg_tick;
   const int32_t* cnt;
   int nseg;
+  int part0;
   long long n_active, S;
 }};
 
@@ -214,14 +304,13 @@ __global__ void __launch_bounds__(KUN_TS_THREADS) {self.kname}(const {pstruct} P
   // ticks so far (capped) and this tick's row in each ring depth
   const int nc = n < (1LL << 30) ? (int)n : (1 << 30);
   (void)nc;
-{ring_pos}
   {T}* __restrict__ st = P.st + s;
   int32_t* __restrict__ si = P.si + s;
   (void)st; (void)si;
-{chr(10).join(decl)}
-{chr(10).join(loads)}
-{body}
-{chr(10).join(stores)}
+  switch (P.part0 + (int)blockIdx.y) {{
+{chr(10).join(cases)}
+  default: break;
+  }}
 }}
 """
         init_src = ""
@@ -251,11 +340,18 @@ __global__ void {self.kname}_initk(const {pstruct} P) {{
   P.st = ({T}*)a->state; P.si = (int32_t*)a->state_i;
   P.seg_off = a->seg_off; P.seg_stock0 = a->seg_stock0; P.seg_tick = (const long long*)a->seg_tick;
   P.nseg = a->nseg; P.n_active = a->n_active; P.S = a->num_stocks; P.cnt = a->seg_count;
+  P.part0 = 0;
   if (a->n_active <= 0) return 0;"""
         launch = f"""
 extern "C" int {self.kname}_launch(const KunGpuStageArgs* a, void* stream) {{
 {common}
-  {self.kname}<<<(unsigned)((a->n_active + KUN_TS_THREADS - 1) / KUN_TS_THREADS), KUN_TS_THREADS, 0, (cudaStream_t)stream>>>(P);
+  // parts [first[k], first[k + 1]) are launch unit k; all of them together
+  // when no unit is asked for
+  static const int first[] = {{{", ".join(str(v) for v in first + [len(parts)])}}};
+  const int k = a->only_kernel - 1;
+  P.part0 = k < 0 ? 0 : first[k];
+  const int n = (k < 0 ? {len(parts)} : first[k + 1]) - P.part0;
+  {self.kname}<<<dim3((unsigned)((a->n_active + KUN_TS_THREADS - 1) / KUN_TS_THREADS), (unsigned)n), KUN_TS_THREADS, 0, (cudaStream_t)stream>>>(P);
   return (int)cudaGetLastError();
 }}
 """
