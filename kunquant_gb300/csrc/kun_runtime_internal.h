@@ -135,6 +135,9 @@ struct Executor {
     void *group_host = nullptr;
     Arena group_dev;
     size_t group_host_bytes = 0;
+    // pinned memory of small host runs (at most kBounceBytes)
+    void *bounce = nullptr;
+    size_t bounce_bytes = 0;
     // copy streams for device-to-host output copies overlapping the stages
     std::vector<cudaStream_t> copy_streams;
     std::vector<cudaEvent_t> copy_ev;    // per stage: its outputs are ready

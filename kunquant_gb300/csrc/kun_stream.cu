@@ -395,6 +395,18 @@ bool stream_order(const KunGpuModuleDesc *m, std::vector<int> &order) {
     return (int)order.size() == m->num_stages;
 }
 
+struct FetchRow {
+    const void *ring;
+    int window;
+};
+// row `tick % window` of every listed ring, one after the other
+template <typename T>
+__global__ void fetch_rows(const FetchRow *__restrict__ rows, T *__restrict__ out, long long S, long long tick) {
+    const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const FetchRow r = rows[blockIdx.y];
+    if (s < S) out[blockIdx.y * S + s] = ((const T *)r.ring)[tick % r.window * S + s];
+}
+
 struct StreamCtx {
     Executor *ex = nullptr;
     const KunGpuModuleDesc *m = nullptr;
@@ -408,13 +420,32 @@ struct StreamCtx {
     std::vector<std::vector<char>> mirror;
     cudaGraphExec_t graph = nullptr;
     TickLevels levels;
+    // Reads of current rows: a program that reads the same few or many
+    // buffers every tick gets them in one copy.  The buffers read since the
+    // last tick, those read between the two ticks before, and (fetched: the
+    // tick they belong to) the latter's rows in pinned memory.
+    std::vector<int> read_now, read_before;
+    std::vector<int> fetch_slot;  // per buffer: its row of the fetched block, or -1
+    std::vector<int> fetch_set;   // buffers of the device table below
+    long long fetched = -1;
+    void *d_fetch = nullptr, *h_fetch = nullptr;
+    FetchRow *d_fetch_rows = nullptr;
     cudaStream_t stream() const { return ex->streams[0]; }
     ~StreamCtx() {
+        release_fetch();
         if (graph) cudaGraphExecDestroy(graph);
         free_tick_levels(levels);
         if (d_seg) cudaFree(d_seg);
         if (d_tick) cudaFree(d_tick);
         store.release();
+    }
+    void release_fetch() {
+        if (d_fetch) cudaFree(d_fetch);
+        if (d_fetch_rows) cudaFree(d_fetch_rows);
+        if (h_fetch) cudaFreeHost(h_fetch);
+        d_fetch = h_fetch = nullptr;
+        d_fetch_rows = nullptr;
+        fetch_set.clear();
     }
 };
 
@@ -751,6 +782,8 @@ static KunStatus ctx_run(StreamCtx *c, bool sync) {
     for (int b = 0; b < m->num_buffers; b++)
         if (m->buffers[b].kind != KUN_BUF_INPUT) c->last_row[b] = (int)(c->tick % win_of(m, b));
     c->tick++;
+    if (!c->read_now.empty()) c->read_before.swap(c->read_now);
+    c->read_now.clear();
     if (sync) {
         e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
@@ -845,12 +878,63 @@ KUN_EXPORT const void *kunStreamGetCurrentBufferDevice(KunStreamContextHandle co
     return (const char *)c->store.rings[h] + (size_t)c->last_row[h] * c->S * elem;
 }
 
+// Brings the rows that were read after the tick before (kFetchMin or more of
+// them, `h` among them) to pinned memory in one copy; false to read `h` alone.
+static constexpr size_t kFetchMin = 4;
+static bool fetch_rows_read_before(StreamCtx *c, int h) {
+    const std::vector<int> &set = c->read_before;
+    if (set.size() < kFetchMin || std::find(set.begin(), set.end(), h) == set.end()) return false;
+    const size_t elem = elem_of(c->m), row = (size_t)c->S * elem;
+    for (int b : set)  // rows of the last tick (an input may have been pushed for the next)
+        if (c->m->buffers[b].kind == KUN_BUF_INPUT || c->last_row[b] != (int)((c->tick - 1) % win_of(c->m, b)))
+            return false;
+    cudaStream_t st = c->stream();
+    if (set != c->fetch_set) {
+        c->release_fetch();
+        std::vector<FetchRow> rows;
+        for (int b : set) rows.push_back({c->store.rings[b], win_of(c->m, b)});
+        if (set.size() > 65535 || cudaMalloc(&c->d_fetch, set.size() * row) != cudaSuccess ||
+            cudaMalloc((void **)&c->d_fetch_rows, rows.size() * sizeof(FetchRow)) != cudaSuccess ||
+            cudaHostAlloc(&c->h_fetch, set.size() * row, cudaHostAllocDefault) != cudaSuccess ||
+            cudaMemcpyAsync(c->d_fetch_rows, rows.data(), rows.size() * sizeof(FetchRow), cudaMemcpyHostToDevice,
+                            st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            cudaGetLastError();
+            c->release_fetch();
+            c->read_before.clear();  // not again before another tick's reads
+            return false;
+        }
+        c->fetch_set = set;
+    }
+    const dim3 grid((unsigned)((c->S + 255) / 256), (unsigned)set.size());
+    if (elem == 4)
+        fetch_rows<<<grid, 256, 0, st>>>(c->d_fetch_rows, (float *)c->d_fetch, c->S, c->tick - 1);
+    else
+        fetch_rows<<<grid, 256, 0, st>>>(c->d_fetch_rows, (double *)c->d_fetch, c->S, c->tick - 1);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(c->h_fetch, c->d_fetch, set.size() * row, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    c->fetch_slot.assign(c->m->num_buffers, -1);
+    for (size_t k = 0; k < set.size(); k++) c->fetch_slot[set[k]] = (int)k;
+    c->fetched = c->tick;
+    return true;
+}
+
 KUN_EXPORT const float *kunStreamGetCurrentBuffer(KunStreamContextHandle context, size_t h) {
     StreamCtx *c = C(context);
     if (!valid_handle(c, h)) return nullptr;
     size_t elem = elem_of(c->m);
     auto &mir = c->mirror[h];
     mir.resize((size_t)c->S * elem);
+    if (std::find(c->read_now.begin(), c->read_now.end(), (int)h) == c->read_now.end()) c->read_now.push_back((int)h);
+    if ((c->fetched == c->tick && c->fetch_slot[h] >= 0) ||
+        (c->read_now.size() == 1 && fetch_rows_read_before(c, (int)h))) {
+        memcpy(mir.data(), (const char *)c->h_fetch + (size_t)c->fetch_slot[h] * mir.size(), mir.size());
+        return (const float *)mir.data();
+    }
     cudaMemcpyAsync(mir.data(), kunStreamGetCurrentBufferDevice(context, h), mir.size(), cudaMemcpyDeviceToHost,
                     c->stream());
     if (cudaStreamSynchronize(c->stream()) != cudaSuccess) {
@@ -870,6 +954,7 @@ static KunStatus push(StreamCtx *c, size_t h, const void *src, cudaMemcpyKind ki
         set_error("push failed: %s", cudaGetErrorString(e));
         return KUN_CUDA_ERROR;
     }
+    if (c->m->buffers[h].kind != KUN_BUF_INPUT) c->fetched = -1;
     c->last_row[h] = row;
     return KUN_SUCCESS;
 }

@@ -427,9 +427,9 @@ class StreamContext:
         p = runtime().kunStreamGetCurrentBuffer(self.handle, handle)
         if not p:
             raise KunError(_err())
-        ct = ctypes.c_float if self._mod.dtype == np.float32 else ctypes.c_double
-        arr = np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ct)), shape=(self.num_stocks,))
-        return arr.copy()
+        arr = np.empty(self.num_stocks, self._mod.dtype)
+        ctypes.memmove(arr.ctypes.data, p, arr.nbytes)
+        return arr
 
     def getCurrentBufferDevice(self, handle: int):
         """The current row of a buffer as a torch CUDA tensor (a copy made on
