@@ -473,8 +473,12 @@ VEC_U = 4
 # rows a thread computes at once in a kernel without window loops, where
 # the rows share no loads and more of them only cost registers
 VEC_U_ELEM = 2
-# rows a window queue loads ahead of use, and the unroll of the window loop
+# rows a window queue loads ahead of use, and the unroll of the loops over
+# windows (10 divides the usual windows: 5 to 20% on a kernel of window sums
+# against 4) and over the common run of window extremes (their branches grow
+# past the instruction cache beyond 4)
 VEC_PREFETCH = 0
+LOOP_UNROLL = 10
 VEC_UNROLL = 4
 # rows a scan loads while it works on as many others (32 rows are a tenth
 # faster alone, but take 255 registers from the kernels beside it)
@@ -1395,7 +1399,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
                         L.append(f"{ind}{T} {qn}[{QL}];")
                         L.append(f"{ind}#pragma unroll")
                         L.append(f"{ind}for (int u = 0; u < {QL}; ++u) {qn}[u] = {self._vload(src, f't + u - {wh - 1}')};")
-                L.append(f"{ind}#pragma unroll {VEC_UNROLL}")
+                L.append(f"{ind}#pragma unroll {LOOP_UNROLL}")
                 L.append(f"{ind}for (int iter = {w - 1}; iter >= {seg}; --iter) {{")
                 bi = ind + "  "
                 L.append(f"{bi}#pragma unroll")
@@ -1704,14 +1708,20 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
 {chr(10).join(self.lines)}
 }}
 """)
-            # kernels with window loops or window states also come compiled for
-            # 64 registers a thread (8 blocks of 128 threads an SM), picked per
-            # kernel by the tuner; elementwise kernels need fewer anyway, and
-            # scan kernels keep one instance
+            # kernels with window loops are held to 72 registers a thread (7
+            # blocks of 128 threads an SM: their chains of dependent sums need the
+            # warps; without a limit they took up to 127 and Alpha158 5000 x 2500
+            # 12.87 ms against 12.48, Alpha101 8192 x 2500 63.4 against 62.1).
+            # They and the kernels with window states also come compiled for 64,
+            # picked per kernel by the tuner; elementwise kernels need fewer
+            # anyway, and scan kernels keep one instance
             if kd["kind"] == "cscan" or (kd["kind"] == "par" and any(
                     ops[i]["k"] in ("ForeachBackWindow", "SkipListState") for i in kd["comp"])):
                 capped.add(ki)
-            for suf, minb in ([("", "KUN_TS_MINB"), ("_r", "8")] if ki in capped else [("", "KUN_TS_MINB")]):
+            loops_only = kd["kind"] == "par" and T == "float" and not any(
+                ops[i]["k"] == "SkipListState" for i in kd["comp"])
+            minb = "7" if ki in capped and loops_only else "KUN_TS_MINB"
+            for suf, minb in [("", minb)] + ([("_r", "8")] if ki in capped else []):
                 srcs.append(f"""__global__ void __launch_bounds__(KUN_TS_THREADS, {minb}) {kname}{suf}(const {pstruct} P) {{
   const int bx = blockIdx.x, by = blockIdx.y;
 {pick}
