@@ -80,6 +80,7 @@ constexpr size_t kSmemOptIn = 40 * 1024;
 // rows 16 us (132), 3000 x 1500 41 us (88), 8192 x 2500 167 us (336), the same
 // with 10 tied values 120 us (530); fp64 801 x 1000 22 us (244).
 constexpr int kRankMaxStocks = 16384;
+constexpr int kRankPad = 4;  // keys behind a row's, for the counting loop's step
 constexpr int kRankPoor = 20;   // counting up to this many neighbours costs less than another map
 constexpr int kRankWorst = 96;  // counting 96 neighbours costs about as much as sorting the row
 
@@ -88,7 +89,7 @@ __host__ __device__ inline int rank_threads(int S, int items) {
     return (w < 1 ? 1 : w) * 32;
 }
 template <typename T> __host__ __device__ inline size_t rank_smem_bytes(int nt, int items) {
-    return (size_t)nt * items * (sizeof(T) + sizeof(uint32_t) + sizeof(uint16_t));
+    return (size_t)nt * items * (sizeof(T) + sizeof(uint32_t) + sizeof(uint16_t)) + kRankPad * sizeof(T);
 }
 
 // register budget (launch bounds): 40 a thread for 8 values in fp32, so that
@@ -133,10 +134,12 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k)
     return k;
 }
 // T(sum) / T(cnt) / T(n) of the equal range [less, less + eq) with the integer
-// rank sum; eq = 1 leaves one division (x / 1 is x).  The sum stays below
-// 2^31: less + eq <= n <= 16384.  The division by the row's n is Markstein's
-// (IBM J. Res. Dev. 34, 1990): with r = 1/n rounded to nearest and a residual
-// by FMA, q + (s - q n) r is the correctly rounded quotient.
+// rank sum (2 less + eq + 1) eq / 2, below 2^31: less + eq <= n <= 16384.  A
+// sum that T holds exactly leaves the mean rank (2 less + eq + 1) / 2 exact, so
+// only larger ones (thousands of ties, in float) need the first division.  The
+// division by the row's n is Markstein's (IBM J. Res. Dev. 34, 1990): with
+// r = 1/n rounded to nearest and a residual by FMA, q + (s - q n) r is the
+// correctly rounded quotient.
 template <typename T> struct RankDivisor;
 template <> struct RankDivisor<float> {
     float n, r;
@@ -160,9 +163,13 @@ template <> struct RankDivisor<double> {
         return __fma_rn(__fma_rn(-q, n, s), r, q);
     }
 };
+template <typename T> __device__ __noinline__ T rank_mean_of_large(uint32_t sum, uint32_t eq) {
+    return kdiv((T)(int)sum, (T)(int)eq);
+}
 template <typename T> __device__ __forceinline__ T rank_value(uint32_t less, uint32_t eq, const RankDivisor<T> &n) {
-    T s = (T)(int)(less + 1);
-    if (eq != 1) s = kdiv((T)(int)((2 * less + eq + 1) * eq / 2), (T)(int)eq);
+    const uint32_t twice = 2 * less + eq + 1, sum2 = twice * eq;
+    T s = kmul((T)(int)twice, T(0.5));
+    if (sizeof(T) == 4 && sum2 > (2u << 24)) s = rank_mean_of_large<T>(sum2 / 2, eq);
     return n(s);
 }
 
@@ -289,7 +296,7 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int B = nt * ITEMS;
     K *rep = reinterpret_cast<K *>(smem), *vals = rep;
-    uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)B * sizeof(K));  // count | unlike << 16
+    uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)(B + kRankPad) * sizeof(K));  // count | unlike << 16
     uint16_t *base = reinterpret_cast<uint16_t *>(hist + B);
     K k[ITEMS];
 #pragma unroll
@@ -425,8 +432,22 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
         rank_row_sorted<T>(row, S, n, nt, reinterpret_cast<K *>(smem), out);
         return;
     }
-    // the representatives are no longer needed: the values unlike them take
-    // their place
+    // The representatives are no longer needed: the values unlike them take
+    // their place, each bucket's from its base on.  The rest is the greatest
+    // key, and later buckets hold greater values, so a bucket's count may run
+    // past its end: four values a step without a test (a loop over exactly the
+    // bucket's took half of all instructions, as a warp's lanes differ).
+    constexpr int WIDE = 16 / sizeof(K);
+    struct alignas(16) Keys {
+        K k[WIDE];
+    };
+    Keys none;
+#pragma unroll
+    for (int q = 0; q < WIDE; q++) none.k[q] = SK::kMax;
+#pragma unroll
+    for (int e = 0; e < ITEMS / WIDE; e++) reinterpret_cast<Keys *>(vals)[e * nt + tid] = none;
+    if (tid < kRankPad) vals[B + tid] = SK::kMax;
+    rank_sync(nt);
 #pragma unroll
     for (int e = 0; e < ITEMS; e++)
         if (pk[e] >> 30) vals[base[pk[e] & 0x3fff] + ((pk[e] >> 14) & 0x3fff)] = k[e];
@@ -440,11 +461,18 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
             uint32_t less = base[at], eq = like;
             if (unlike) {
                 uint32_t same = 0;
+                const K *v = vals + less, *end = v + unlike;
 #pragma unroll 1
-                for (uint32_t p = less, p1 = less + unlike; p < p1; p++) {
-                    const K y = vals[p];
-                    less += (y < k[e]);
-                    same += (y == k[e]);
+                for (; v < end; v += 4) {
+                    const K y0 = v[0], y1 = v[1], y2 = v[2], y3 = v[3];
+                    less += (y0 < k[e]);
+                    same += (y0 == k[e]);
+                    less += (y1 < k[e]);
+                    same += (y1 == k[e]);
+                    less += (y2 < k[e]);
+                    same += (y2 == k[e]);
+                    less += (y3 < k[e]);
+                    same += (y3 == k[e]);
                 }
                 if (pk[e] >> 30) eq = same;
                 if (pk[e] >> 31) less += like;
