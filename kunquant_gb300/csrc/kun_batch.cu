@@ -58,7 +58,7 @@ struct BatchRun {
 // are numbered alike in every job's part of the arena, and the kernels are
 // weighed by the jobs' summed cells.  Null when the module or memory has none.
 static const Plan *batch_node_plan(Executor *ex, const KunGpuModuleDesc *m, const std::vector<BatchJob> &jobs) {
-    const int ns = (int)ex->streams.size();
+    const int ns = node_streams(ex);
     if (ns < 2 || jobs.size() < 2) return nullptr;
     long long cells = 0, rows = 0;
     size_t slot_bytes = 0;
@@ -404,7 +404,8 @@ KUN_EXPORT KunStatus kunRunGraphBatch(KunExecutorHandle exec, KunModuleHandle mo
     int64_t launches = 0;
     if (br.nodes) {
         if ((rs = batch_nodes(br, st, launches)) != KUN_SUCCESS) {
-            for (cudaStream_t q : ex->streams) cudaStreamSynchronize(q);  // kernels enqueued so far use the buffers
+            for (auto *list : {&ex->streams, &ex->extra_streams})
+                for (cudaStream_t q : *list) cudaStreamSynchronize(q);  // kernels enqueued so far use the buffers
             return rs;
         }
     }

@@ -102,6 +102,7 @@ struct GraphEntry {
 struct Executor {
     int device = 0;
     std::vector<cudaStream_t> streams;
+    std::vector<cudaStream_t> extra_streams;  // of plans in kernels (node_streams)
     cudaStream_t user_stream = nullptr;
     Arena arena;
     Arena staging;
@@ -147,6 +148,10 @@ struct Executor {
     // they were made (call with `mu` held)
     void check_epoch();
 };
+
+// Streams a plan in kernels may use: 1 for a single-stream executor, else at
+// least kNodeStreams, the missing ones created here.
+int node_streams(Executor *ex);
 
 // Launches a plan's nodes on the executor's streams, forked from and joined to
 // `origin` (its stream 0): launch(place, node, stream), until it returns false.
