@@ -62,14 +62,15 @@ constexpr size_t kSmemOptIn = 40 * 1024;
 //     (logarithmic in the value) for rows of one sign crowded towards zero.
 //     The first value of a bucket is its representative.
 //  3. The counters are scanned; a value that differs from its bucket's
-//     representative takes a place among such values.  Where there is none
-//     the scan alone gives the ranks, so ties cost nothing, however many.
-//  4. Those values are scattered by bucket, and every value of their buckets
-//     counts the smaller and equal ones among them.
+//     representative takes a place among those below or above it.  The others'
+//     ranks are then known, so ties cost nothing, however many.
+//  4. Those values are scattered by bucket and side, and each counts the
+//     smaller and equal ones on its side.
 //
-// When a bucket holds more than kRankPoor values unlike its representative,
-// the map is refined (rank_refine), then the other map is tried and refined; a row that none of the four spreads is sorted
-// in shared memory (rank_row_sorted).  Bound by the issue rate: about 235
+// When more than kRankPoor values of a bucket lie on one side (sides are
+// counted in 8 bits, which kRankWorst stays below), the map is refined
+// (rank_refine), then the other map is tried and refined; a row that none of the
+// four spreads is sorted in shared memory (rank_row_sorted).  Bound by the issue rate: about 190
 // instructions a value with 75% of the issue slots taken at 8192 stocks, so the
 // block is as small as the row allows and several rows share an SM: 8 values a
 // thread up to 4096 stocks and 16 above.  Shared memory: B keys
@@ -296,7 +297,8 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int B = nt * ITEMS;
     K *rep = reinterpret_cast<K *>(smem), *vals = rep;
-    uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)(B + kRankPad) * sizeof(K));  // count | unlike << 16
+    // count | below the representative << 16 | above << 24
+    uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)(B + kRankPad) * sizeof(K));
     uint16_t *base = reinterpret_cast<uint16_t *>(hist + B);
     K k[ITEMS];
 #pragma unroll
@@ -390,9 +392,11 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
         for (int e = 0; e < ITEMS; e++) {
             const K r = rep[pk[e]];
             if (k[e] != SK::kMax && r != k[e]) {
-                const uint32_t place = atomicAdd(&hist[pk[e]], 0x10000u) >> 16;
+                const bool below = k[e] < r;
+                const uint32_t old = atomicAdd(&hist[pk[e]], below ? 1u << 16 : 1u << 24);
+                const uint32_t place = below ? (old >> 16) & 0xff : old >> 24;
                 deep = max(deep, place);
-                pk[e] |= place << 14 | (k[e] < r ? 1u << 30 : 2u << 30);
+                pk[e] |= place << 14 | (below ? 1u << 30 : 2u << 30);
             }
         }
         // exclusive scan of the counts, ITEMS consecutive ones a thread
@@ -426,17 +430,22 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
             break;
         }
         // a bucket that most of the row is in asks for the other map at once
-        if (attempt == 0 && rank_sync_or(nt, deep >= (uint32_t)n / 4 * 3)) attempt = 1;
+        if (attempt == 0) {
+            uint32_t crowd = 0;
+#pragma unroll
+            for (int e = 0; e < ITEMS; e++) crowd = max(crowd, hist[pk[e] & 0x3fff] & 0xffff);
+            if (rank_sync_or(nt, crowd >= (uint32_t)n / 4 * 3)) attempt = 1;
+        }
     }
     if (sorted) {
         rank_row_sorted<T>(row, S, n, nt, reinterpret_cast<K *>(smem), out);
         return;
     }
     // The representatives are no longer needed: the values unlike them take
-    // their place, each bucket's from its base on.  The rest is the greatest
-    // key, and later buckets hold greater values, so a bucket's count may run
-    // past its end: four values a step without a test (a loop over exactly the
-    // bucket's took half of all instructions, as a warp's lanes differ).
+    // their place, in each bucket's part those below from its start on and those
+    // above towards its end.  The rest is the greatest key, and later buckets
+    // hold greater values, so a count may run past its list: four values a step
+    // without a test (a warp's lanes have lists of unlike length).
     constexpr int WIDE = 16 / sizeof(K);
     struct alignas(16) Keys {
         K k[WIDE];
@@ -450,32 +459,36 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
     rank_sync(nt);
 #pragma unroll
     for (int e = 0; e < ITEMS; e++)
-        if (pk[e] >> 30) vals[base[pk[e] & 0x3fff] + ((pk[e] >> 14) & 0x3fff)] = k[e];
+        if (pk[e] >> 30) {
+            const int at = pk[e] & 0x3fff, place = (pk[e] >> 14) & 0xff;
+            vals[base[at] + ((pk[e] >> 31) ? (int)(hist[at] & 0xffff) - 1 - place : place)] = k[e];
+        }
     rank_sync(nt);
 #pragma unroll
     for (int e = 0; e < ITEMS; e++) {
         const int i = e * nt + tid;
         if (i < S) {
             const int at = pk[e] & 0x3fff;
-            const uint32_t w = hist[at], unlike = w >> 16, like = (w & 0xffff) - unlike;
-            uint32_t less = base[at], eq = like;
-            if (unlike) {
-                uint32_t same = 0;
-                const K *v = vals + less, *end = v + unlike;
+            const uint32_t w = hist[at], cnt = w & 0xffff, below = (w >> 16) & 0xff, above = w >> 24;
+            // a value like the representative has all below and none above
+            uint32_t less = base[at] + below, eq = cnt - below - above;
+            if (pk[e] >> 30) {
+                const bool up = pk[e] >> 31;
+                less = up ? less + eq : less - below;  // where its list starts
+                eq = 0;
+                const K *v = vals + less, *end = v + (up ? above : below);
 #pragma unroll 1
                 for (; v < end; v += 4) {
                     const K y0 = v[0], y1 = v[1], y2 = v[2], y3 = v[3];
                     less += (y0 < k[e]);
-                    same += (y0 == k[e]);
+                    eq += (y0 == k[e]);
                     less += (y1 < k[e]);
-                    same += (y1 == k[e]);
+                    eq += (y1 == k[e]);
                     less += (y2 < k[e]);
-                    same += (y2 == k[e]);
+                    eq += (y2 == k[e]);
                     less += (y3 < k[e]);
-                    same += (y3 == k[e]);
+                    eq += (y3 == k[e]);
                 }
-                if (pk[e] >> 30) eq = same;
-                if (pk[e] >> 31) less += like;
             }
             out(i, k[e] != SK::kMax ? rank_value<T>(less, eq, over_n) : knan<T>());
         }
