@@ -1060,7 +1060,7 @@ class LeveledGen(StageGen):
             # the registers for the window sums (single-buffered)
             return SLIDE_BLOCK
         if any(ops[i]["k"] == "WindowedLinearRegression" for i in role["comp"]):
-            return SCAN_BLOCK // 2
+            return SCAN_BLOCK // 4
         return SCAN_BLOCK if n <= 4 else (8 if n <= 8 else 4)
 
     def _scan_prefetch(self, role: dict, B: int, ind: str, chunk: bool = False):
@@ -1191,7 +1191,51 @@ class LeveledGen(StageGen):
         def args(pre):
             return "".join(f"{pre}{x}, " for x in arrays)
 
+        # a regression and its outputs alone: the sums of all rows first, then
+        # every row's quotients as straight-line code, and again with kdiv for
+        # a block where an operand was out of DivFast's range
+        regs = [i for i in comp if ops[i]["k"] == "WindowedLinearRegression"]
+        outs = [i for i in sorted(comp) if ops[i]["k"] in LR_CONS]
+        lone = (T == "float" and self.RT == "float" and len(regs) == 1 and len(outs) + 1 == len(comp)
+                and set(stores) <= set(outs) and all(ops[i]["in"][0] == regs[0] for i in outs))
+
+        def regression(guard):
+            r = regs[0]
+            src, w = ops[r]["in"][0], ops[r]["window"]
+            shared = "true" if contraction.regression_shares_square(ops, r) else "false"
+            L.append(f"{bi}kun::LinSums<{T}> ls[{B}];")
+            L.append(f"{bi}#pragma unroll")
+            L.append(f"{bi}for (int u = 0; u < {B}; ++u) {{")
+            L.append(f"{bj}lr{r}.template step<{shared}>({wins[(src, str(w))]}[u], pv{src}[u]);")
+            L.append(f"{bj}ls[u] = lr{r}.sums();")
+            L.append(f"{bi}}}")
+
+            def quotients(div):
+                L.append(f"{bj}#pragma unroll")
+                L.append(f"{bj}for (int u = 0; u < {B}; ++u) {{")
+                if guard:
+                    L.append(f"{bj}  if (tb + u >= length) break;")
+                for i in outs:
+                    fn = {"WindowedLinearRegressionRSqaureImpl": f"rsq({div})",
+                          "WindowedLinearRegressionSlopeImpl": f"slope({div})"}.get(ops[i]["k"])
+                    if fn is None:
+                        fn = f"resi(pv{ops[i]['in'][1]}[u], {float(w)!r}f, {div})"
+                    if i in stores:
+                        L.append(f"{bj}  b{i}[(tb + u) * st{i}] = ls[u].{fn};")
+                L.append(f"{bj}}}")
+
+            L.append(f"{bi}kun::DivFast div;")
+            L.append(f"{bi}{{")
+            quotients("div")
+            L.append(f"{bi}}}")
+            L.append(f"{bi}if (!div.ok) {{")
+            quotients("kun::DivRn()")
+            L.append(f"{bi}}}")
+
         def steps(guard):
+            if lone:
+                regression(guard)
+                return
             L.append(f"{bi}#pragma unroll")
             L.append(f"{bi}for (int u = 0; u < {B}; ++u) {{")
             L.append(f"{bj}const long long t = tb + u;")
