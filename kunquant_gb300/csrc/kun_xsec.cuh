@@ -69,8 +69,9 @@ constexpr size_t kSmemOptIn = 40 * 1024;
 //
 // When more than kRankPoor values of a bucket lie on one side (sides are
 // counted in 8 bits, which kRankWorst stays below), the map is refined
-// (rank_refine), then the other map is tried and refined; a row that none of the
-// four spreads is sorted in shared memory (rank_row_sorted).  Bound by the issue rate: about 190
+// (rank_refine), at most twice (correlations of ranks a few units in the last
+// place around zero need it), then the other map is; a row that none of them
+// spreads is sorted in shared memory (rank_row_sorted).  Bound by the issue rate: about 190
 // instructions a value with 75% of the issue slots taken at 8192 stocks, so the
 // block is as small as the row allows and several rows share an SM: 8 values a
 // thread up to 4096 stocks and 16 above.  Shared memory: B keys
@@ -370,11 +371,11 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
                                     __popc(__ballot_sync(0xffffffffu, from < spread * 0.0625f)) >= 20);
     uint32_t pk[ITEMS];  // bucket | place << 14 | relation to the representative << 30 (1 below, 2 above)
     bool sorted = false;
-    for (int attempt = 0;; attempt++) {
-        if (attempt & 1) {
+    for (int attempt = 0;; attempt++) {  // a map, refined, refined again; then the other
+        if (attempt % 3) {
             rank_refine<T, ITEMS>(k, pk, nt, hist, base, rep);
         } else {
-            const RankMap<T> map(wide || key_first != (attempt == 2), lo, hi, B);
+            const RankMap<T> map(wide || key_first != (attempt == 3), lo, hi, B);
 #pragma unroll
             for (int e = 0; e < ITEMS; e++) pk[e] = (uint32_t)rank_swizzle(map(k[e]));
         }
@@ -424,8 +425,8 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
             run = b3 + (q.w & 0xffff);
             reinterpret_cast<uint2 *>(base)[sw] = make_uint2(b0 | b1 << 16, b2 | b3 << 16);
         }
-        if (!rank_sync_or(nt, deep >= (uint32_t)(attempt < 3 ? kRankPoor : kRankWorst))) break;
-        if (attempt == 3) {
+        if (!rank_sync_or(nt, deep >= (uint32_t)(attempt < 5 ? kRankPoor : kRankWorst))) break;
+        if (attempt == 5) {
             sorted = true;
             break;
         }
@@ -434,7 +435,7 @@ __device__ __forceinline__ void rank_row(const T *__restrict__ row, int S, int n
             uint32_t crowd = 0;
 #pragma unroll
             for (int e = 0; e < ITEMS; e++) crowd = max(crowd, hist[pk[e] & 0x3fff] & 0xffff);
-            if (rank_sync_or(nt, crowd >= (uint32_t)n / 4 * 3)) attempt = 1;
+            if (rank_sync_or(nt, crowd >= (uint32_t)n / 4 * 3)) attempt = 2;
         }
     }
     if (sorted) {
