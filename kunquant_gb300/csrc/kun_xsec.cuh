@@ -71,7 +71,7 @@ constexpr size_t kSmemOptIn = 40 * 1024;
 // counted in 8 bits, which kRankWorst stays below), the map is refined
 // (rank_refine), at most twice (correlations of ranks a few units in the last
 // place around zero need it), then the other map is; a row that none of them
-// spreads is sorted in shared memory (rank_row_sorted).  Bound by the issue rate: about 190
+// spreads is sorted in shared memory (rank_row_sorted).  Bound by the issue rate: about 220
 // instructions a value with 75% of the issue slots taken at 8192 stocks, so the
 // block is as small as the row allows and several rows share an SM: 8 values a
 // thread up to 4096 stocks and 16 above.  Shared memory: B keys
@@ -79,8 +79,8 @@ constexpr size_t kSmemOptIn = 40 * 1024;
 // scanned counts, 10 bytes a value in fp32.  Normal values, against a bitonic
 // network in 1024-thread blocks up to 1024 stocks and, above, buckets with a
 // radix sort behind them in one 1024-thread block an SM: 997 stocks x 1251
-// rows 16 us (132), 3000 x 1500 41 us (88), 8192 x 2500 167 us (336), the same
-// with 10 tied values 120 us (530); fp64 801 x 1000 22 us (244).
+// rows 16 us (132), 3000 x 1500 37 us (88), 8192 x 2500 156 us (336), the same
+// with 10 tied values 125 us (530); fp64 801 x 1000 23 us (244).
 constexpr int kRankMaxStocks = 16384;
 constexpr int kRankPad = 4;  // keys behind a row's, for the counting loop's step
 constexpr int kRankPoor = 20;   // counting up to this many neighbours costs less than another map
