@@ -264,7 +264,9 @@ __device__ __forceinline__ void rank_refine(const typename SortKey<T>::K (&k)[IT
 
 // The bucket maps of a row, 1 .. B - 2 for finite values, monotone over all:
 // -inf is 0, +inf the last or beside the greatest.  In float for both types
-// (rounding to float is monotone, and FP64 arithmetic is slow here).
+// (rounding to float is monotone, and FP64 arithmetic is slow here).  The shift
+// brings the finite values' key distances to 32 bits; that of a double's +inf
+// may have more, and counts as the greatest.
 template <typename T> struct RankMap {
     using SK = SortKey<T>;
     using K = typename SK::K;
@@ -273,6 +275,10 @@ template <typename T> struct RankMap {
     float scale, top;
     K lo;
     T vlo;
+    static __device__ __forceinline__ uint32_t saturate(uint32_t d) { return d; }
+    static __device__ __forceinline__ uint32_t saturate(unsigned long long d) {
+        return d >> 32 ? 0xffffffffu : (uint32_t)d;
+    }
     __device__ __forceinline__ RankMap(bool by_key_, K lo_, K hi, int B) : by_key(by_key_), lo(lo_), vlo(SK::dec(lo_)) {
         shift = SK::bits(hi - lo) > 32 ? SK::bits(hi - lo) - 32 : 0;
         const float range = by_key ? __uint2float_rn((uint32_t)((hi - lo) >> shift)) : (float)ksub(SK::dec(hi), vlo);
@@ -280,7 +286,7 @@ template <typename T> struct RankMap {
         scale = fminf(__fdiv_rn((float)(B - 3), range), 3e38f);  // finite: 0 * scale is 0
     }
     __device__ __forceinline__ int operator()(K k) const {
-        const float d = by_key ? (k < lo ? -1.f : __uint2float_rn((uint32_t)((k - lo) >> shift)))
+        const float d = by_key ? (k < lo ? -1.f : __uint2float_rn(saturate((k - lo) >> shift)))
                                : (float)ksub(SK::dec(k), vlo);
         return (int)fminf(fmaxf(__fmul_rn(d, scale), -1.f), top) + 1;
     }
