@@ -26,7 +26,7 @@
 
 namespace kungpu {
 
-constexpr int kCorrThreads = 128;
+constexpr int kCorrThreads = 256;
 
 // element (t, s) of a [T][S] (layout 1) or [S/L][T][L] (layout 0) buffer
 __device__ __forceinline__ long long util_index(int layout, long long s, long long t, long long S, long long T,
@@ -34,20 +34,20 @@ __device__ __forceinline__ long long util_index(int layout, long long s, long lo
     return layout == 1 ? t * S + s : (s / L) * T * L + t * L + s % L;
 }
 
-// Sums of a thread, all kept as unnormalised pairs (kun::df_acc).  A sum that
-// has left the finite range is its high part alone: the pair's error term is
-// then NaN.
+// Sums of a thread, normalised at every addition: values far from zero leave
+// the correlation only what the sums hold beyond float (left unnormalised, their
+// low parts' rounding made its error 1.8 to 2.8 times as large at 15000 stocks).
 template <int N> struct CorrSums {
     kun::DFloat v[N];
-    // one more value of every thread's sums over the block's first nt threads;
-    // thread 0 has the totals
+    // every thread's sums over the block's first nt threads: a butterfly in each
+    // warp, then the warps in order; thread 0 has the totals
     __device__ __forceinline__ void reduce(int nt) {
         __shared__ float sh[N][2][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = nt >> 5;
 #pragma unroll
         for (int q = 0; q < N; q++) {
-            if (!isfinite(v[q].hi)) v[q].lo = 0.f;
-            v[q] = warp_sum(v[q]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[q] = kun::kadd(v[q], across(v[q], lane ^ o));
             if (lane == 0) {
                 sh[q][0][w] = v[q].hi;
                 sh[q][1][w] = v[q].lo;
@@ -55,19 +55,14 @@ template <int N> struct CorrSums {
         }
         __syncthreads();
         if (w == 0) {
+            kun::DFloat total;  // lane q adds sum q
+            for (int i = 0; i < nw && lane < N; i++) total = kun::kadd(total, kun::DFloat(sh[lane][0][i], sh[lane][1][i]));
 #pragma unroll
-            for (int q = 0; q < N; q++)
-                v[q] = warp_sum(lane < nw ? kun::DFloat(sh[q][0][lane], sh[q][1][lane]) : kun::DFloat());
+            for (int q = 0; q < N; q++) v[q] = across(total, q);
         }
     }
-    static __device__ __forceinline__ kun::DFloat warp_sum(kun::DFloat x) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const kun::DFloat y(__shfl_xor_sync(0xffffffffu, x.hi, o), __shfl_xor_sync(0xffffffffu, x.lo, o));
-            kun::df_acc_pair(x, y);
-            if (!isfinite(x.hi)) x.lo = 0.f;
-        }
-        return x;
+    static __device__ __forceinline__ kun::DFloat across(kun::DFloat x, int from) {
+        return kun::DFloat(__shfl_sync(0xffffffffu, x.hi, from), __shfl_sync(0xffffffffu, x.lo, from));
     }
 };
 
@@ -78,8 +73,8 @@ __global__ void __launch_bounds__(kCorrThreads) corr_label_rows(const float *__r
     CorrSums<2> a;
     for (long long s = threadIdx.x; s < S; s += blockDim.x) {
         const float b = y[util_index(layout, s, t, S, T, L)];
-        kun::df_acc(a.v[0], b);
-        kun::df_acc_prod(a.v[1], b, b);
+        a.v[0] = kun::df_add_f(a.v[0], b);
+        a.v[1] = kun::df_add_prod(a.v[1], b, b);
     }
     a.reduce(blockDim.x);
     if (threadIdx.x == 0) ysum[t] = make_float4(a.v[0].hi, a.v[0].lo, a.v[1].hi, a.v[1].lo);
@@ -90,9 +85,9 @@ struct CorrRow {
     float x[2], x2[2], xy[2];
 };
 __device__ __forceinline__ void corr_add(CorrSums<3> &a, float x, float y) {
-    kun::df_acc(a.v[0], x);
-    kun::df_acc_prod(a.v[1], x, x);
-    kun::df_acc_prod(a.v[2], x, y);
+    a.v[0] = kun::df_add_f(a.v[0], x);
+    a.v[1] = kun::df_add_prod(a.v[1], x, x);
+    a.v[2] = kun::df_add_prod(a.v[2], x, y);
 }
 __device__ __forceinline__ void corr_store(const CorrSums<3> &a, CorrRow *o) {
     *o = CorrRow{{a.v[0].hi, a.v[0].lo}, {a.v[1].hi, a.v[1].lo}, {a.v[2].hi, a.v[2].lo}};
