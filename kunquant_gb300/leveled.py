@@ -1619,6 +1619,10 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
         tma_src: List[str] = []
         capped: Set[int] = set()  # kernels with a 64-register instance
         warm: Dict[int, int] = {}  # rows a tile runs before its own
+        # chunked scans restart their sums at every tile, so their rounding follows
+        # it: one tile for all sizes, or a universe's results would depend on the
+        # stocks, days and universes beside it
+        fixed: Set[int] = set()
         knames = []
         pstruct = f"P_{self.kname}"
         for ki, kd in enumerate(ks):
@@ -1698,7 +1702,7 @@ __global__ void __launch_bounds__(128) {kname}_tma(const {pstruct} P) {{
                 self.lines += self._moment_decls("  ")
                 self._scan_prefetch(r, self._scan_block(r), "  ", chunk=True)
                 kinfo.append((max(64, (2 * wmax + 15) // 16 * 16), 0))
-                warm[ki] = wmax
+                fixed.add(ki)
             else:
                 roles = kd["roles"]
                 self.lines.append("  switch (by) {")
@@ -1804,7 +1808,8 @@ struct {pstruct} {{
             if not sc:
                 tuned = f"(a->tune_tile && a->tune_tile[{k}] > 0)"
                 sel.append(f"  P.tile[{k}] = {tuned} ? a->tune_tile[{k}] : {d};")
-                sel.append(f"  if (!{tuned}) P.tile[{k}] = kun::pick_tile(a, 1, P.tile[{k}], {warm[k]}, blk{k});")
+                if k not in fixed:
+                    sel.append(f"  if (!{tuned}) P.tile[{k}] = kun::pick_tile(a, 1, P.tile[{k}], {warm[k]}, blk{k});")
             else:
                 sel.append(f"  P.tile[{k}] = 0;")
         for k, (d, sc) in enumerate(kinfo):
@@ -1825,7 +1830,7 @@ struct {pstruct} {{
                 calls.append(f"  {knames[k]}<<<{grid}>>>(P);")
             calls.append("  if (cudaError_t e = cudaGetLastError()) return (int)e;\n  }")
         launch = self.launcher(pstruct, "\n".join(sel + calls))
-        launch += self._group_launcher(pstruct, knames, kinfo, capped, warm)
+        launch += self._group_launcher(pstruct, knames, kinfo, capped, warm, fixed)
         return head + "".join(srcs) + "".join(tma_src), launch
 
     def _kernel_io(self, kd: dict) -> List[int]:
@@ -1859,7 +1864,7 @@ struct {pstruct} {{
         return [int(cost), len(reads)] + sorted(reads) + [len(writes)] + sorted(writes)
 
     def _group_launcher(self, pstruct: str, knames: List[str], kinfo, capped: Set[int],
-                        warm: Dict[int, int]) -> str:
+                        warm: Dict[int, int], fixed: Set[int]) -> str:
         """prepare(): the parameter blocks of n jobs; launch_group(): every
         kernel of the stage once over all jobs' tiles."""
         fill = "\n".join(f"    P.p[{sl}] = a->buffers[{bid}];" for bid, sl in self.slots.items())
@@ -1870,16 +1875,17 @@ struct {pstruct} {{
                 tiles.append(f"    P.tile[{k}] = 0;")
                 continue
             # one tile for the group, from all its jobs' rows
+            pick = str(d) if k in fixed else f"kun::pick_tile(args, njobs, {d}, {warm[k]}, tb & 0xffff)"
             picks.append(f"  int tile{k};\n  {{\n    const KunGpuStageArgs* a = &args[0];\n"
                          f"    const int tb = (a->tune_block && a->tune_block[{k}] > 0) ? a->tune_block[{k}] : KUN_TS_THREADS;\n"
-                         f"    tile{k} = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : "
-                         f"kun::pick_tile(args, njobs, {d}, {warm[k]}, tb & 0xffff);\n  }}")
+                         f"    (void)tb;\n"
+                         f"    tile{k} = (a->tune_tile && a->tune_tile[{k}] > 0) ? a->tune_tile[{k}] : {pick};\n  }}")
             tiles.append(f"    P.tile[{k}] = tile{k};")
         launches = []
         for k, (d, sc) in enumerate(kinfo):
             gy = str(d) if sc else f"(a->length + tile - 1) / tile"
-            tl = ("0" if sc else f"(args[0].tune_tile && args[0].tune_tile[{k}] > 0) ? args[0].tune_tile[{k}] : "
-                  f"kun::pick_tile(args, njobs, {d}, {warm[k]}, blk)")
+            pick = str(d) if sc or k in fixed else f"kun::pick_tile(args, njobs, {d}, {warm[k]}, blk)"
+            tl = "0" if sc else f"(args[0].tune_tile && args[0].tune_tile[{k}] > 0) ? args[0].tune_tile[{k}] : {pick}"
             kcall = (f"{knames[k]}_grp<<<(unsigned)total, blk, 0, (cudaStream_t)stream>>>((const {pstruct}*)dev, tt);"
                      if k not in capped else
                      f"if (tb & KUN_BLOCK_REGCAP) {knames[k]}_r_grp<<<(unsigned)total, blk, 0, (cudaStream_t)stream>>>"
