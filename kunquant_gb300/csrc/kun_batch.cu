@@ -417,15 +417,13 @@ KUN_EXPORT KunStatus kunRunGraphBatch(KunExecutorHandle exec, KunModuleHandle mo
         cudaStreamWaitEvent(st, ex->bridge_in, 0);
     }
     int64_t launches = 0;
-    if (br.nodes) {
-        if ((rs = batch_nodes(br, st, launches)) != KUN_SUCCESS) {
-            for (auto *list : {&ex->streams, &ex->extra_streams})
-                for (cudaStream_t q : *list) cudaStreamSynchronize(q);  // kernels enqueued so far use the buffers
-            return rs;
-        }
-    }
+    if (br.nodes) rs = batch_nodes(br, st, launches);
     for (int si : br.order)
-        if (!br.nodes && (rs = batch_stage(br, si, st, nullptr, nullptr, launches)) != KUN_SUCCESS) return rs;
+        if (!br.nodes && rs == KUN_SUCCESS) rs = batch_stage(br, si, st, nullptr, nullptr, launches);
+    if (rs != KUN_SUCCESS) {
+        drain(ex);
+        return rs;
+    }
     ex->last_launches = launches;
     return batch_finish(ex, st, synchronize != 0);
 }
@@ -452,6 +450,10 @@ KUN_EXPORT int kunExecutorTune(KunExecutorHandle exec, KunModuleHandle mod, int 
     if (batch_setup(ex, m, njobs, (const NameMap *const *)buffers, num_stocks, total_time, cur_time, length, false,
                     br) != KUN_SUCCESS)
         return -1;
+    struct AtEnd {  // also where a stage's launch fails
+        Executor *ex;
+        ~AtEnd() { drain(ex); }
+    } at_end{ex};
     reps = std::max(1, reps);
     const int tiles[] = {0, 16, 32, 64, 128, 256};
     const int blocks[] = {64, 128};

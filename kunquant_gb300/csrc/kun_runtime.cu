@@ -387,6 +387,16 @@ int node_slots(const Plan &p) {
 // host buffers of a run up to which they go through pinned memory
 static constexpr size_t kBounceBytes = 64u << 20;
 
+void drain(Executor *ex) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ex->stream(), &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;
+    }
+    for (auto *list : {&ex->streams, &ex->extra_streams, &ex->copy_streams})
+        for (cudaStream_t q : *list) cudaStreamSynchronize(q);
+}
+
 KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &names, long long S,
                     long long total_time, long long cur_time, long long length, bool sync) {
     clear_error();
@@ -523,6 +533,10 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
     gkey.push_back((void *)(intptr_t)nstreams);
     KunStatus rs = KUN_SUCCESS;
     GraphEntry *ge = nullptr;
+    auto failed = [&](KunStatus status) {
+        drain(ex);
+        return status;
+    };
     // host outputs: copy each one out as soon as its stage is done (no graph
     // replay for such runs; the copies are not part of the captured work)
     OutputCopies oc;
@@ -561,7 +575,7 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
     }
     if (overlap) {
         rs = enqueue_stages(ex, m, plan, ptrs.data(), S, total_time, cur_time, length, st, multi, launches, &oc);
-        if (rs != KUN_SUCCESS) return rs;
+        if (rs != KUN_SUCCESS) return failed(rs);
         for (size_t k = 0; k < ex->copy_streams.size(); k++) {
             cudaEventRecord(ex->copy_done[k], ex->copy_streams[k]);
             cudaStreamWaitEvent(st, ex->copy_done[k], 0);
@@ -597,7 +611,7 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
                     cudaGetLastError();
                 }
                 if (g) cudaGraphDestroy(g);
-                if (rs != KUN_SUCCESS) return rs;
+                if (rs != KUN_SUCCESS) return failed(rs);
             }
         }
     }
@@ -607,12 +621,12 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
         cudaError_t e = cudaGraphLaunch(ge->exec, st);
         if (e != cudaSuccess) {
             set_error("graph launch failed: %s", cudaGetErrorString(e));
-            return KUN_CUDA_ERROR;
+            return failed(KUN_CUDA_ERROR);
         }
         launches = ge->launches;
     } else {
         rs = enqueue_stages(ex, m, plan, ptrs.data(), S, total_time, cur_time, length, st, multi, launches);
-        if (rs != KUN_SUCCESS) return rs;
+        if (rs != KUN_SUCCESS) return failed(rs);
     }
     ex->last_launches = launches;
     bool had_host_out = overlap || !host_out.empty();

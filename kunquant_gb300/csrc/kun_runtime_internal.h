@@ -153,6 +153,11 @@ struct Executor {
 // least kNodeStreams, the missing ones created here.
 int node_streams(Executor *ex);
 
+// After a launch that failed: waits for the kernels and copies enqueued before
+// it, which use the arena, the staging and the caller's buffers and which
+// nothing joins any more.  (Under a caller's capture nothing has run.)
+void drain(Executor *ex);
+
 // Launches a plan's nodes on the executor's streams, forked from and joined to
 // `origin` (its stream 0): launch(place, node, stream), until it returns false.
 void run_nodes(Executor *ex, const Plan &plan, cudaStream_t origin,
