@@ -684,8 +684,7 @@ Executor *create_executor(int nstreams) {
     return ex;
 }
 
-void destroy_executor(Executor *ex) {
-    if (!ex) return;
+static void destroy_executor(Executor *ex) {
     for (auto *list : {&ex->streams, &ex->extra_streams})
         for (auto s : *list) {
             cudaStreamSynchronize(s);
@@ -709,6 +708,10 @@ void destroy_executor(Executor *ex) {
     delete ex;
 }
 
+void drop_executor(Executor *ex) {
+    if (ex && ex->holders.fetch_sub(1) == 1) destroy_executor(ex);
+}
+
 }  // namespace kungpu
 
 using namespace kungpu;
@@ -717,7 +720,7 @@ static const KunGpuModuleDesc *M(KunModuleHandle m) { return (const KunGpuModule
 
 KUN_EXPORT KunExecutorHandle kunCreateSingleThreadExecutor(void) { return create_executor(1); }
 KUN_EXPORT KunExecutorHandle kunCreateMultiThreadExecutor(int numthreads) { return create_executor(numthreads); }
-KUN_EXPORT void kunDestoryExecutor(KunExecutorHandle ptr) { destroy_executor((Executor *)ptr); }
+KUN_EXPORT void kunDestoryExecutor(KunExecutorHandle ptr) { drop_executor((Executor *)ptr); }
 
 KUN_EXPORT KunLibraryHandle kunLoadLibrary(const char *path_or_name) {
     clear_error();

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <functional>
 #include <map>
 #include <memory>
@@ -100,6 +101,10 @@ struct GraphEntry {
 };
 
 struct Executor {
+    // the caller's handle, and every stream context and serving pool made on it:
+    // the last to go frees it, for handles are destroyed in any order (at a
+    // program's end, for one)
+    std::atomic<int> holders{1};
     int device = 0;
     std::vector<cudaStream_t> streams;
     std::vector<cudaStream_t> extra_streams;  // of plans in kernels (node_streams)
@@ -147,6 +152,23 @@ struct Executor {
     // drops plans, graphs and tuned shapes if a library was unloaded since
     // they were made (call with `mu` held)
     void check_epoch();
+};
+
+void drop_executor(Executor *ex);  // one holder less; the last one frees it
+// what a stream context or a serving pool holds its executor by
+class ExecutorRef {
+    Executor *ex_ = nullptr;
+
+  public:
+    ExecutorRef() = default;
+    ExecutorRef(const ExecutorRef &) = delete;
+    ExecutorRef &operator=(const ExecutorRef &) = delete;
+    ~ExecutorRef() { drop_executor(ex_); }
+    void hold(Executor *ex) {
+        ex->holders.fetch_add(1);
+        ex_ = ex;
+    }
+    Executor *operator->() const { return ex_; }
 };
 
 // Streams a plan in kernels may use: 1 for a single-stream executor, else at

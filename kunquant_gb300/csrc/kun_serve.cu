@@ -83,7 +83,7 @@ struct Session {
 };
 
 struct ServePool {
-    Executor *ex = nullptr;
+    ExecutorRef ex;
     const KunGpuModuleDesc *m = nullptr;
     long long cap = 0;
     int max_sessions = 0;
@@ -440,7 +440,7 @@ KUN_EXPORT KunStatus kunCreateServePool(KunExecutorHandle exec, KunModuleHandle 
     }
     cudaSetDevice(ex->device);
     std::unique_ptr<ServePool> p(new ServePool());
-    p->ex = ex;
+    p->ex.hold(ex);
     p->m = m;
     p->cap = (long long)capacity_stocks;
     p->max_sessions = max_sessions;

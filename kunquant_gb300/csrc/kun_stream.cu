@@ -408,7 +408,7 @@ __global__ void fetch_rows(const FetchRow *__restrict__ rows, T *__restrict__ ou
 }
 
 struct StreamCtx {
-    Executor *ex = nullptr;
+    ExecutorRef ex;
     const KunGpuModuleDesc *m = nullptr;
     long long S = 0;
     long long tick = 0;
@@ -718,7 +718,7 @@ static StreamCtx *create_ctx(Executor *ex, const KunGpuModuleDesc *m, long long 
     }
     cudaSetDevice(ex->device);
     auto *c = new StreamCtx();
-    c->ex = ex;
+    c->ex.hold(ex);
     c->m = m;
     c->S = S;
     rc = KUN_OUT_OF_MEMORY;
