@@ -91,7 +91,7 @@ struct ServePool {
     StreamStore store;
     std::vector<int> order;
     std::vector<int> in_bufs, out_bufs;
-    // device: segment table {off[max+1], stock0[max], cnt[3]} then ticks,
+    // device: segment table {off[max+1], stock0[max], cnt[4]} then ticks,
     // ring pointer/window arrays, input/output tables by column
     char *d_table = nullptr;
     char *h_table = nullptr;  // pinned mirror
@@ -239,7 +239,7 @@ static KunStatus run_step(ServePool *p, const StepShape &sh, const void *dev_in,
     cudaStream_t st = p->stream();
     size_t elem = p->elem();
     // the table goes as two copies: ints up to cnt, then the ticks
-    cudaMemcpyAsync(p->d_table, p->h_table, (2 * p->max_sessions + 4) * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(p->d_table, p->h_table, (2 * p->max_sessions + 5) * sizeof(int32_t), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(p->d_table + p->tick_off, p->h_table + p->tick_off, sh.nsess * sizeof(long long),
                     cudaMemcpyHostToDevice, st);
     // every input and output row moves as 2D copies: one over the column
@@ -314,6 +314,9 @@ static KunStatus prepare_step(ServePool *p, int nsess, const int64_t *sids, std:
         s.stamp = stamp;
         sel[k] = &s;
     }
+    // the sessions of Rank's long rows come first, cnt[3] of them
+    const auto short_ones = std::stable_partition(
+        sel.begin(), sel.end(), [](const Session *q) { return q->len > (long long)kun::kRankShort; });
     for (int k = 0; k < nsess; k++) {
         Session &s = *sel[k];
         off[k] = (int32_t)n;
@@ -341,6 +344,7 @@ static KunStatus prepare_step(ServePool *p, int nsess, const int64_t *sids, std:
     cnt[0] = nsess;
     cnt[1] = (int32_t)n;
     cnt[2] = longest;
+    cnt[3] = (int32_t)(short_ones - sel.begin());
     sh.nsess = nsess;
     sh.n = n;
     sh.lo = lo;
@@ -459,7 +463,7 @@ KUN_EXPORT KunStatus kunCreateServePool(KunExecutorHandle exec, KunModuleHandle 
         if (m->buffers[b].kind == KUN_BUF_OUTPUT) p->out_bufs.push_back(b);
     }
     size_t elem = p->elem();
-    size_t ints = (size_t)(2 * max_sessions + 4);
+    size_t ints = (size_t)(2 * max_sessions + 5);
     p->tick_off = (ints * sizeof(int32_t) + 15) / 16 * 16;
     p->table_bytes = p->tick_off + (size_t)max_sessions * sizeof(long long);
     size_t nin = p->in_bufs.size(), nout = p->out_bufs.size();

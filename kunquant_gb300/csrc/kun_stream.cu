@@ -298,29 +298,49 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
                        const TickLevels *levels) {
     const KunGpuModuleDesc *m = store.m;
     if (levels && levels->ok) {
+        // Rank over a device table's segments: a launch for the short ones beside
+        // one for the long ones, of which the step's stocks allow a few only.  A
+        // block with the threads and shared memory of the longest segment fills
+        // an SM whatever it ranks (256 sessions of 64 stocks in a pool that takes
+        // 16384: 1140 us a step in one launch, 594 in two).
+        // (A pool for longer rows than Rank takes is refused whatever its step.)
+        const int longest = max_len > kun::kRankMaxStocks ? max_len : (int)std::min<long long>(max_len, n_active);
+        const bool both = d_seg_count && longest > kun::kRankShort;
         for (size_t l = 0; l < levels->other.size(); l++) {
             // the level's first launch stays on the tick's stream
             const auto &units = levels->other[l];
-            const size_t here = levels->rank_cnt[l] > 0 ? 0 : 1;
-            const size_t sides = std::min(units.size() > here ? units.size() - here : 0, levels->side.size());
+            const bool ranks = levels->rank_cnt[l] > 0, two = ranks && both;
+            const size_t here = ranks ? 0 : 1;
+            const size_t beside = (units.size() > here ? units.size() - here : 0) + two;
+            const size_t sides = std::min(beside, levels->side.size());
             if (sides) cudaEventRecord(levels->fork, st);
             for (size_t k = 0; k < sides; k++) cudaStreamWaitEvent(levels->side[k], levels->fork, 0);
             for (size_t u = 0; u < units.size(); u++) {
-                cudaStream_t on = u < here || !sides ? st : levels->side[(u - here) % sides];
+                cudaStream_t on = u < here || !sides ? st : levels->side[(u - here + two) % sides];
                 KunStatus rs = launch_stage(store, units[u].stage, units[u].kernel, d_seg_off, d_seg_stock0, d_tick,
                                             nseg, n_active, max_len, on, d_seg_count);
                 if (rs != KUN_SUCCESS) return rs;
             }
-            if (levels->rank_cnt[l] > 0) {
+            if (ranks) {
                 const kun::RankJob *jobs = (const kun::RankJob *)levels->d_jobs + levels->rank_off[l];
-                int rc = m->dtype == 0
-                             ? kun::launch_rank_multi_segments<float>(jobs, levels->rank_cnt[l], store.cap, d_seg_off,
-                                                                      d_seg_stock0, (const long long *)d_tick, nseg,
-                                                                      max_len, d_seg_count, st)
-                             : kun::launch_rank_multi_segments<double>(jobs, levels->rank_cnt[l], store.cap,
-                                                                       d_seg_off, d_seg_stock0,
-                                                                       (const long long *)d_tick, nseg, max_len,
-                                                                       d_seg_count, st);
+                auto launch = [&](int segs, int len, kun::RankPart part, cudaStream_t on) {
+                    return m->dtype == 0
+                               ? kun::launch_rank_multi_segments<float>(jobs, levels->rank_cnt[l], store.cap, d_seg_off,
+                                                                        d_seg_stock0, (const long long *)d_tick, segs,
+                                                                        len, d_seg_count, part, on)
+                               : kun::launch_rank_multi_segments<double>(jobs, levels->rank_cnt[l], store.cap,
+                                                                         d_seg_off, d_seg_stock0,
+                                                                         (const long long *)d_tick, segs, len,
+                                                                         d_seg_count, part, on);
+                };
+                int rc = 0;
+                if (two) {
+                    rc = launch(nseg, kun::kRankShort, kun::kRankShortOnes, levels->side[0]);
+                    const int most = (int)std::min<long long>(nseg, n_active / (kun::kRankShort + 1) + 1);
+                    if (!rc) rc = launch(most, longest, kun::kRankLongOnes, st);
+                } else {
+                    rc = launch(nseg, longest, kun::kRankAll, st);
+                }
                 if (rc) {
                     set_error("rank stages of level %d failed: %s", (int)l, cudaGetErrorString((cudaError_t)rc));
                     return KUN_CUDA_ERROR;

@@ -546,13 +546,19 @@ __global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_se
                                  smem_raw);
 }
 
+// A step's table lists its segments of more than kRankShort stocks first and
+// holds their number in cnt[3]; a launch takes those, the others, or all.
+constexpr int kRankShort = 1024;
+enum RankPart { kRankAll, kRankLongOnes, kRankShortOnes };
+
 template <typename T, int ITEMS, int MAXT>
 __global__ void __launch_bounds__(MAXT, rank_min_blocks<T>(ITEMS, MAXT)) rank_multi_segments(const RankJob *__restrict__ jobs, long long cap,
                                                             const int32_t *seg_off, const int32_t *seg_stock0,
-                                                            const long long *seg_tick, const int32_t *cnt) {
+                                                            const long long *seg_tick, const int32_t *cnt,
+                                                            RankPart part) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int k = blockIdx.x;
-    if (cnt && k >= cnt[0]) return;
+    if (cnt && (k >= cnt[0] || (part != kRankAll && (k < cnt[3]) != (part == kRankLongOnes)))) return;
     const RankJob jb = jobs[blockIdx.y];
     rank_segment<T, ITEMS, MAXT>((const T *)jb.in, jb.w_in, (T *)jb.out, jb.w_out, cap, seg_off[k + 1] - seg_off[k],
                                  seg_stock0[k], seg_tick[k], smem_raw);
@@ -834,12 +840,12 @@ inline int launch_rank_segments(const T *in, int w_in, T *out, int w_out, long l
     });
 }
 
-// njobs Rank stages over the step's segments in one launch (cnt: the step's
-// device table, or null when the step has exactly nseg segments)
+// njobs Rank stages over (a part of) the step's segments in one launch (cnt:
+// the step's device table, or null when the step has exactly nseg segments)
 template <typename T>
 inline int launch_rank_multi_segments(const RankJob *d_jobs, int njobs, long long cap, const int32_t *seg_off,
                                       const int32_t *seg_stock0, const long long *seg_tick, int nseg, int max_len,
-                                      const int32_t *cnt, cudaStream_t st) {
+                                      const int32_t *cnt, RankPart part, cudaStream_t st) {
     if (njobs <= 0 || nseg <= 0) return 0;
     if (njobs > 65535) return (int)cudaErrorInvalidValue;
     return rank_dispatch<true>(max_len, [&](auto items, auto maxt) {
@@ -848,7 +854,7 @@ inline int launch_rank_multi_segments(const RankJob *d_jobs, int njobs, long lon
         const size_t smem = rank_smem_bytes<T>(nt, I);
         if (int e = rank_smem_limit(rank_multi_segments<T, I, M>, smem)) return e;
         rank_multi_segments<T, I, M><<<dim3((unsigned)nseg, (unsigned)njobs), nt, smem, st>>>(
-            d_jobs, cap, seg_off, seg_stock0, seg_tick, cnt);
+            d_jobs, cap, seg_off, seg_stock0, seg_tick, cnt, part);
         return (int)cudaGetLastError();
     });
 }
