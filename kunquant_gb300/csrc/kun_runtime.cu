@@ -170,13 +170,15 @@ bool make_plan(const KunGpuModuleDesc *m, long long S, long long length, int nst
     return true;
 }
 
-static bool is_device_pointer(const void *ptr) {
+enum class Memory { kDevice, kPinned, kPageable };
+static Memory memory_of(const void *ptr) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, ptr) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return Memory::kPageable;
     }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    if (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) return Memory::kDevice;
+    return a.type == cudaMemoryTypeHost ? Memory::kPinned : Memory::kPageable;
 }
 
 static size_t user_buffer_elems(const KunGpuModuleDesc *m, const KunGpuBufferDesc &b, long long S,
@@ -384,8 +386,26 @@ int node_slots(const Plan &p) {
     return p.num_slots + (int)std::min<size_t>(spare, (size_t)p.num_slots);
 }
 
-// host buffers of a run up to which they go through pinned memory
-static constexpr size_t kBounceBytes = 64u << 20;
+// Runs on host buffers of up to kReplayBytes in all are replayed as one graph
+// between their copies (the staging's addresses stay); larger ones copy every
+// output as it is ready.  Pageable buffers then go through pinned memory of the
+// executor's in one copy each way.  That saves some 15 us a buffer for its own
+// copy and 2 us a kernel for its launch, and costs a copy by the host, 1 us for 13
+// KB: where their bytes are worth more, such a run is as a large one.  Pinned
+// buffers are copied as they are.  Replayed and not, us on 8 streams: Alpha101 (88
+// buffers, 564 kernels) 64 x 260 pageable 955 and 3270, pinned 725 and 2265, 300 x
+// 260 pageable 2617 and 3572, 450 x 300 4228 and 3706; Alpha158 (163 and 147) 150
+// x 260 pageable 2307 and 3300, 300 x 300 4760 and 3567, pinned 1219 and 1199; one
+// Rank of 3000 x 700 pageable 1168 and 165.
+static constexpr size_t kReplayBytes = 64u << 20;
+static constexpr size_t kBounceBuffer = 192u << 10;  // bytes that a buffer's copy is worth
+static constexpr size_t kBounceKernel = 24u << 10;   // and a kernel's launch
+
+static size_t num_kernels(const KunGpuModuleDesc *m) {
+    size_t n = 0;
+    for (int i = 0; i < m->num_stages; i++) n += m->stages[i].num_kernels > 0 ? m->stages[i].num_kernels : 1;
+    return n;
+}
 
 void drain(Executor *ex) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -460,6 +480,7 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
         void *host;
         size_t bytes;
         size_t off;
+        bool pinned;
     };
     std::vector<HostCopy> host_in, host_out;
     for (int b = 0; b < m->num_buffers; b++) {
@@ -474,35 +495,42 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
             set_error("Buffer name not found: %s", bd.name);
             return KUN_INVALID_ARGUMENT;
         }
-        if (is_device_pointer(f->second)) {
+        const Memory where = memory_of(f->second);
+        if (where == Memory::kDevice) {
             ptrs[b] = f->second;
         } else {
-            HostCopy hc{b, f->second, user_buffer_elems(m, bd, S, total_time, length) * elem, 0};
+            HostCopy hc{b, f->second, user_buffer_elems(m, bd, S, total_time, length) * elem, 0,
+                        where == Memory::kPinned};
             (bd.kind == KUN_BUF_INPUT ? host_in : host_out).push_back(hc);
         }
     }
-    size_t staging_in = 0, staging_need = 0;
-    for (auto *list : {&host_in, &host_out}) {
-        for (auto &hc : *list) {
+    // their places in the staging: pageable inputs, pageable outputs, the pinned
+    size_t staging_need = 0, bounce_in = 0, bounce_need = 0, pageable = 0;
+    auto place = [&](std::vector<HostCopy> &list, bool pinned) {
+        for (auto &hc : list) {
+            if (hc.pinned != pinned) continue;
             hc.off = staging_need;
             staging_need += align_up(hc.bytes, 256);
+            pageable += !pinned;
         }
-        if (list == &host_in) staging_in = staging_need;
-    }
-    // Small host runs go through pinned memory with one copy each way, their
-    // kernels replayed as one graph (the staging's addresses stay); a copy a
-    // buffer and a launch a kernel took 3.1 ms for 88 buffers of 64 x 260,
-    // where the kernels take 1.  Large ones copy every output as it is ready.
-    bool bounce = staging_need > 0 && staging_need <= kBounceBytes && !ex->profile;
-    if (bounce && ex->bounce_bytes < staging_need) {
+    };
+    place(host_in, false);
+    bounce_in = staging_need;
+    place(host_out, false);
+    bounce_need = staging_need;
+    place(host_in, true);
+    place(host_out, true);
+    bool replay = staging_need > 0 && staging_need <= kReplayBytes && !ex->profile &&
+                  bounce_need <= pageable * kBounceBuffer + num_kernels(m) * kBounceKernel;
+    if (replay && ex->bounce_bytes < bounce_need) {
         if (ex->bounce) cudaFreeHost(ex->bounce);
         ex->bounce = nullptr;
         ex->bounce_bytes = 0;
-        if (cudaHostAlloc(&ex->bounce, staging_need, cudaHostAllocDefault) == cudaSuccess) {
-            ex->bounce_bytes = staging_need;
+        if (cudaHostAlloc(&ex->bounce, bounce_need, cudaHostAllocDefault) == cudaSuccess) {
+            ex->bounce_bytes = bounce_need;
         } else {
             cudaGetLastError();
-            bounce = false;
+            replay = false;
         }
     }
     if (staging_need) {
@@ -512,13 +540,13 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
         }
         for (auto &hc : host_in) {
             ptrs[hc.buf] = (char *)ex->staging.ptr + hc.off;
-            if (bounce)
+            if (replay && !hc.pinned)
                 memcpy((char *)ex->bounce + hc.off, hc.host, hc.bytes);
             else
                 cudaMemcpyAsync(ptrs[hc.buf], hc.host, hc.bytes, cudaMemcpyHostToDevice, st);
         }
-        if (bounce && staging_in)
-            cudaMemcpyAsync(ex->staging.ptr, ex->bounce, staging_in, cudaMemcpyHostToDevice, st);
+        if (replay && bounce_in)
+            cudaMemcpyAsync(ex->staging.ptr, ex->bounce, bounce_in, cudaMemcpyHostToDevice, st);
         for (auto &hc : host_out) ptrs[hc.buf] = (char *)ex->staging.ptr + hc.off;
     }
     int64_t launches = 0;
@@ -540,7 +568,7 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
     // host outputs: copy each one out as soon as its stage is done (no graph
     // replay for such runs; the copies are not part of the captured work)
     OutputCopies oc;
-    bool overlap = !host_out.empty() && !ex->profile && !bounce;
+    bool overlap = !host_out.empty() && !ex->profile && !replay;
     if (overlap) {
         if (ex->copy_streams.empty()) {
             for (int k = 0; k < 4; k++) {
@@ -630,11 +658,11 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
     }
     ex->last_launches = launches;
     bool had_host_out = overlap || !host_out.empty();
-    if (bounce && staging_need > staging_in)
-        cudaMemcpyAsync((char *)ex->bounce + staging_in, (char *)ex->staging.ptr + staging_in,
-                        staging_need - staging_in, cudaMemcpyDeviceToHost, st);
+    if (replay && bounce_need > bounce_in)
+        cudaMemcpyAsync((char *)ex->bounce + bounce_in, (char *)ex->staging.ptr + bounce_in, bounce_need - bounce_in,
+                        cudaMemcpyDeviceToHost, st);
     for (auto &hc : host_out)
-        if (!bounce) cudaMemcpyAsync(hc.host, ptrs[hc.buf], hc.bytes, cudaMemcpyDeviceToHost, st);
+        if (!replay || hc.pinned) cudaMemcpyAsync(hc.host, ptrs[hc.buf], hc.bytes, cudaMemcpyDeviceToHost, st);
     if (ex->has_user_stream) {
         cudaEventRecord(ex->bridge_out, st);
         cudaStreamWaitEvent(ex->user_stream, ex->bridge_out, 0);
@@ -646,7 +674,7 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
             return KUN_CUDA_ERROR;
         }
         for (auto &hc : host_out)
-            if (bounce) memcpy(hc.host, (const char *)ex->bounce + hc.off, hc.bytes);
+            if (replay && !hc.pinned) memcpy(hc.host, (const char *)ex->bounce + hc.off, hc.bytes);
         if (ex->d_error) {
             // a kernel whose bounded wait for a bulk copy ran out (never
             // expected: a hardware or launch-setup fault) reports it here

@@ -141,7 +141,7 @@ struct Executor {
     void *group_host = nullptr;
     Arena group_dev;
     size_t group_host_bytes = 0;
-    // pinned memory of small host runs (at most kBounceBytes)
+    // pinned memory that small pageable buffers go through (at most kReplayBytes)
     void *bounce = nullptr;
     size_t bounce_bytes = 0;
     // copy streams for device-to-host output copies overlapping the stages
