@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from kunquant_gb300 import runner as kr
+from oracle import utils as U
 
 F = np.float32
 THREADS = 256
@@ -80,3 +81,28 @@ def test_sums_of_values_far_from_zero(layout, S, ratio):
     # on values ratio^2 times the variances, fused or not
     tol = 2.0 ** -24 + 8 * ratio * ratio * 2.0 ** -53
     assert np.abs(out - _restated(x, y)).max() <= tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S", [40, 997, 5000, 8193, 15000])
+@pytest.mark.parametrize("ratio", [0, 1e3, 1e5])
+def test_sums_of_ranks(S, ratio):
+    """The ranks' sums hold far more than the result shows; what the label's
+    distance from zero leaves is the restated label sums'."""
+    rng = np.random.default_rng(S + 1)
+    T = 24
+    n = rng.standard_normal((T, S))
+    x = np.floor(8 * n).astype(F) if S < 1000 else n.astype(F)
+    y = (ratio + 0.5 * n + rng.standard_normal((T, S))).astype(F)
+    out = np.empty(T, F)
+    kr.corrWith(kr.createSingleThreadExecutor(), [x], y, [out], rank_inputs=True)
+    r = np.stack([U._rank_row(row) for row in x]).astype(np.float64)
+    p = y.astype(np.float64) ** 2
+    hi = p.astype(F)
+    my, my2 = _sum(y, np.zeros_like(y)) / S, _sum(hi, (p - hi).astype(F)) / S
+    mx, mx2, mxy = r.sum(1) / S, (r * r).sum(1) / S, (r * (y - ratio)).sum(1) / S + ratio * r.sum(1) / S
+    want = (mxy - mx * my) / (np.sqrt(mx2 - mx * mx) * np.sqrt(my2 - my * my))
+    # the result's rounding, that of the double moments (the label's second one
+    # ratio^2 times its variance), and of sums of ratio * S / 2 in two floats
+    tol = 2.0 ** -24 + 8 * ratio * ratio * 2.0 ** -53 + 8 * (ratio + 1) * 2.0 ** -46
+    assert np.abs(out - want).max() <= tol
