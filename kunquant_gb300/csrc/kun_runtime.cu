@@ -713,7 +713,7 @@ Executor *create_executor(int nstreams) {
 }
 
 static void destroy_executor(Executor *ex) {
-    for (auto *list : {&ex->streams, &ex->extra_streams})
+    for (auto *list : {&ex->streams, &ex->extra_streams, &ex->side})
         for (auto s : *list) {
             cudaStreamSynchronize(s);
             cudaStreamDestroy(s);
@@ -731,6 +731,8 @@ static void destroy_executor(Executor *ex) {
     }
     if (ex->group_host) cudaFreeHost(ex->group_host);
     if (ex->bounce) cudaFreeHost(ex->bounce);
+    for (auto e : ex->side_join) cudaEventDestroy(e);
+    if (ex->side_fork) cudaEventDestroy(ex->side_fork);
     for (auto e : ex->copy_ev) cudaEventDestroy(e);
     for (auto e : ex->copy_done) cudaEventDestroy(e);
     delete ex;

@@ -148,6 +148,11 @@ struct Executor {
     std::vector<cudaStream_t> copy_streams;
     std::vector<cudaEvent_t> copy_ev;    // per stage: its outputs are ready
     std::vector<cudaEvent_t> copy_done;  // per copy stream: all copies issued so far are done
+    // what ticks are captured on beside streams[0] (the graphs do not keep it,
+    // so all contexts and pools share it; made with the first of them)
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> side_join;
+    cudaEvent_t side_fork = nullptr;
     cudaStream_t stream() const { return streams[0]; }
     // drops plans, graphs and tuned shapes if a library was unloaded since
     // they were made (call with `mu` held)
@@ -221,7 +226,8 @@ void free_tick_schedule(TickSchedule &s);
 // stages) and the cross-sectional stages whose longest path from a source has
 // d of them, so those of a level do not depend on each other.  The Rank
 // stages of a level run as one launch over (segment, stage) blocks; the units
-// run beside it on `side`, forked from and joined to the tick's stream.
+// run beside it on the executor's side streams, forked from and joined to the
+// tick's stream.
 struct TickLevels {
     struct Unit {
         int stage, kernel;  // kernel -1: the whole stage
@@ -229,13 +235,11 @@ struct TickLevels {
     std::vector<std::vector<Unit>> other;  // per level: all but the Rank stages
     std::vector<int> rank_off, rank_cnt;   // per level: slice of the job table
     void *d_jobs = nullptr;                // device RankJob table
-    std::vector<cudaStream_t> side;
-    std::vector<cudaEvent_t> join;
-    cudaEvent_t fork = nullptr;
+    const Executor *ex = nullptr;          // whose side streams the units are captured on
     bool ok = false;
 };
 // false when a Rank stage does not read and write exactly one ring
-bool make_tick_levels(const StreamStore &store, const std::vector<int> &order, TickLevels &lv);
+bool make_tick_levels(Executor *ex, const StreamStore &store, const std::vector<int> &order, TickLevels &lv);
 void free_tick_levels(TickLevels &lv);
 
 // Enqueue one tick of every stage of `store` for the segments described by

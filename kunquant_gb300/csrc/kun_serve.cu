@@ -485,7 +485,7 @@ KUN_EXPORT KunStatus kunCreateServePool(KunExecutorHandle exec, KunModuleHandle 
     memset(p->h_table, 0, p->table_bytes);
     // a module whose Rank stages do not fit the level form keeps the
     // stage-by-stage schedule
-    if (!make_tick_levels(p->store, p->order, p->levels)) {
+    if (!make_tick_levels(ex, p->store, p->order, p->levels)) {
         cudaGetLastError();
         free_tick_levels(p->levels);
     }

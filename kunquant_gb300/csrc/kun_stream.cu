@@ -182,7 +182,22 @@ void free_tick_schedule(TickSchedule &s) {
 // into `st`) with events for the cross-stream dependencies.
 static constexpr int kSideStreams = 7;  // launches of a level beside the tick's stream
 
-bool make_tick_levels(const StreamStore &store, const std::vector<int> &order, TickLevels &lv) {
+static bool make_side_streams(Executor *ex) {
+    std::lock_guard<std::mutex> lk(ex->mu);
+    while ((int)ex->side.size() < kSideStreams) {
+        cudaStream_t q;
+        if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) return false;
+        ex->side.push_back(q);
+    }
+    while (ex->side_join.size() < ex->side.size()) {
+        cudaEvent_t e;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
+        ex->side_join.push_back(e);
+    }
+    return ex->side_fork || cudaEventCreateWithFlags(&ex->side_fork, cudaEventDisableTiming) == cudaSuccess;
+}
+
+bool make_tick_levels(Executor *ex, const StreamStore &store, const std::vector<int> &order, TickLevels &lv) {
     const KunGpuModuleDesc *m = store.m;
     // depth of every unit from the depths of the values it reads
     std::vector<int> made(m->num_buffers, -1);  // level that writes the buffer
@@ -239,27 +254,14 @@ bool make_tick_levels(const StreamStore &store, const std::vector<int> &order, T
             cudaSuccess)
             return false;
     }
-    lv.side.assign(kSideStreams, nullptr);
-    lv.join.assign(kSideStreams, nullptr);
-    for (int k = 0; k < kSideStreams; k++)
-        if (cudaStreamCreateWithFlags(&lv.side[k], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&lv.join[k], cudaEventDisableTiming) != cudaSuccess)
-            return false;
-    if (cudaEventCreateWithFlags(&lv.fork, cudaEventDisableTiming) != cudaSuccess) return false;
+    if (!make_side_streams(ex)) return false;
+    lv.ex = ex;
     lv.ok = true;
     return true;
 }
 
 void free_tick_levels(TickLevels &lv) {
     if (lv.d_jobs) cudaFree(lv.d_jobs);
-    for (auto q : lv.side)
-        if (q) cudaStreamDestroy(q);
-    for (auto e : lv.join)
-        if (e) cudaEventDestroy(e);
-    if (lv.fork) cudaEventDestroy(lv.fork);
-    lv.side.clear();
-    lv.join.clear();
-    lv.fork = nullptr;
     lv.d_jobs = nullptr;
     lv.ok = false;
 }
@@ -306,17 +308,18 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
         // (A pool for longer rows than Rank takes is refused whatever its step.)
         const int longest = max_len > kun::kRankMaxStocks ? max_len : (int)std::min<long long>(max_len, n_active);
         const bool both = d_seg_count && longest > kun::kRankShort;
+        const auto &side = levels->ex->side;
         for (size_t l = 0; l < levels->other.size(); l++) {
             // the level's first launch stays on the tick's stream
             const auto &units = levels->other[l];
             const bool ranks = levels->rank_cnt[l] > 0, two = ranks && both;
             const size_t here = ranks ? 0 : 1;
             const size_t beside = (units.size() > here ? units.size() - here : 0) + two;
-            const size_t sides = std::min(beside, levels->side.size());
-            if (sides) cudaEventRecord(levels->fork, st);
-            for (size_t k = 0; k < sides; k++) cudaStreamWaitEvent(levels->side[k], levels->fork, 0);
+            const size_t sides = std::min(beside, side.size());
+            if (sides) cudaEventRecord(levels->ex->side_fork, st);
+            for (size_t k = 0; k < sides; k++) cudaStreamWaitEvent(side[k], levels->ex->side_fork, 0);
             for (size_t u = 0; u < units.size(); u++) {
-                cudaStream_t on = u < here || !sides ? st : levels->side[(u - here + two) % sides];
+                cudaStream_t on = u < here || !sides ? st : side[(u - here + two) % sides];
                 KunStatus rs = launch_stage(store, units[u].stage, units[u].kernel, d_seg_off, d_seg_stock0, d_tick,
                                             nseg, n_active, max_len, on, d_seg_count);
                 if (rs != KUN_SUCCESS) return rs;
@@ -335,7 +338,7 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
                 };
                 int rc = 0;
                 if (two) {
-                    rc = launch(nseg, kun::kRankShort, kun::kRankShortOnes, levels->side[0]);
+                    rc = launch(nseg, kun::kRankShort, kun::kRankShortOnes, side[0]);
                     const int most = (int)std::min<long long>(nseg, n_active / (kun::kRankShort + 1) + 1);
                     if (!rc) rc = launch(most, longest, kun::kRankLongOnes, st);
                 } else {
@@ -347,8 +350,8 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
                 }
             }
             for (size_t k = 0; k < sides; k++) {
-                cudaEventRecord(levels->join[k], levels->side[k]);
-                cudaStreamWaitEvent(st, levels->join[k], 0);
+                cudaEventRecord(levels->ex->side_join[k], side[k]);
+                cudaStreamWaitEvent(st, levels->ex->side_join[k], 0);
             }
         }
         return KUN_SUCCESS;
@@ -755,7 +758,7 @@ static StreamCtx *create_ctx(Executor *ex, const KunGpuModuleDesc *m, long long 
         delete c;
         return nullptr;
     }
-    if (!make_tick_levels(c->store, c->order, c->levels)) {
+    if (!make_tick_levels(ex, c->store, c->order, c->levels)) {
         cudaGetLastError();
         free_tick_levels(c->levels);
     }
