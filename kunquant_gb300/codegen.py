@@ -592,11 +592,12 @@ extern "C" int {self.kname}_launch(const KunGpuStageArgs* a, void* stream) {{
         return src + launch, len(self.scratch), nk
 
 
-def stage_generator(spec: dict, si: int, tag: str, mode: str = "leveled") -> StageGen:
-    """Leveled kernels where the stage allows them, else the single-scan form."""
+def stage_generator(spec: dict, si: int, tag: str, mode: str = "leveled", groups=None) -> StageGen:
+    """Leveled kernels where the stage allows them, else the single-scan form;
+    of a stream module the tick kernels (`groups`: its tick_groups)."""
     if spec["output_layout"] == "STREAM":
         from .streamgen import StreamGen
-        return StreamGen(spec, si, tag)
+        return StreamGen(spec, si, tag, groups)
     if mode == "leveled" and spec["stages"][si]["kind"] == "ts":
         from .leveled import LeveledGen, Unsupported
         try:
@@ -655,8 +656,12 @@ template <> struct LogTables<{T}> {{
     imax: Dict[int, List[int]] = {}
     files: List[List[str]] = []
     cur: List[str] = []
+    groups = None
+    if spec["output_layout"] == "STREAM":
+        from .streamgen import tick_groups
+        groups = tick_groups(spec)
     for si in range(n_stages):
-        g = stage_generator(spec, si, tag, mode)
+        g = stage_generator(spec, si, tag, mode, groups)
         src, nscr, nk = g.generate()
         scratch_counts[si] = nscr
         kernel_counts[si] = nk

@@ -66,16 +66,10 @@ def stage_parts(ops: List[dict]) -> List[List[int]]:
     return sorted(parts.values())
 
 
-_plans: List[tuple] = []
-
-
 def tick_groups(spec: dict) -> Dict[int, List[List[List[int]]]]:
     """Per time-series stage its parts in groups of equal depth, the depth of a
     part being the longest chain of parts and cross-sectional stages before
     it: the parts of one depth, of all stages, do not depend on each other."""
-    for known, groups in _plans:
-        if known is spec:
-            return groups
     nodes = []  # (stage, part or None, reads, writes)
     for si, st in enumerate(spec["stages"]):
         if st["kind"] != "ts":
@@ -98,9 +92,7 @@ def tick_groups(spec: dict) -> Dict[int, List[List[List[int]]]]:
     for k, (si, part, _, _) in enumerate(nodes):
         if part is not None:
             by_stage.setdefault(si, {}).setdefault(depth_of(k), []).append(part)
-    groups = {si: [by_stage[si][d] for d in sorted(by_stage[si])] for si in by_stage}
-    _plans[:] = _plans[-7:] + [(spec, groups)]
-    return groups
+    return {si: [by_stage[si][d] for d in sorted(by_stage[si])] for si in by_stage}
 
 
 class StreamGen(StageGen):
@@ -110,8 +102,9 @@ class StreamGen(StageGen):
     walked all of a stage's windows took up to 100 us of a tick, and the
     stages' chain 39 levels where the parts' has 10."""
 
-    def __init__(self, spec: dict, si: int, tag: str):
+    def __init__(self, spec: dict, si: int, tag: str, groups: Dict[int, List[List[List[int]]]] = None):
         super().__init__(spec, si, tag)
+        self.groups = tick_groups(spec) if groups is None else groups
         self.fplan = contraction.plan(self.ops) if self.st["kind"] == "ts" else {}
         self.state_t_vars = 0
         self.state_i_vars = 0
@@ -225,7 +218,7 @@ class StreamGen(StageGen):
             self.state_i_max += [-1 if f.startswith(("ix[", "idx[")) else W for f in inf]
         self.has_init = bool(fields)
         # ops of one tick (CodegenCpp.py:189-307 with length 1), part by part
-        groups = tick_groups(self.spec)[self.si]
+        groups = self.groups[self.si]
         parts = [part for group in groups for part in group]
         loops = self._loops()
         cases = []
