@@ -80,18 +80,24 @@ def tick_groups(spec: dict) -> Dict[int, List[List[List[int]]]]:
             reads = {ops[j]["buf"] for i in part for j in ops[i]["in"] if ops[j]["k"] == "Input"}
             nodes.append((si, part, reads, {ops[i]["buf"] for i in part if ops[i]["k"] == "Output"}))
     writer = {b: k for k, node in enumerate(nodes) for b in node[3]}
+    before = [{writer[b] for b in node[2] if b in writer and writer[b] != k} for k, node in enumerate(nodes)]
     depth: Dict[int, int] = {}
-
-    def depth_of(k):
-        if k not in depth:
-            depth[k] = max([depth_of(writer[b]) + 1 for b in nodes[k][2] if b in writer and writer[b] != k],
-                           default=0)
-        return depth[k]
-
+    for root in range(len(nodes)):
+        stack = [root]
+        while stack:  # a node's depth once those before it have theirs
+            k = stack[-1]
+            missing = [j for j in before[k] if j not in depth]
+            if missing:
+                stack += missing
+                if len(stack) > len(nodes) * len(nodes) + 1:
+                    raise RuntimeError("cyclic stage graph")
+                continue
+            depth[k] = max([depth[j] + 1 for j in before[k]], default=0)
+            stack.pop()
     by_stage: Dict[int, Dict[int, list]] = {}
     for k, (si, part, _, _) in enumerate(nodes):
         if part is not None:
-            by_stage.setdefault(si, {}).setdefault(depth_of(k), []).append(part)
+            by_stage.setdefault(si, {}).setdefault(depth[k], []).append(part)
     return {si: [by_stage[si][d] for d in sorted(by_stage[si])] for si in by_stage}
 
 

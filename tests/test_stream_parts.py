@@ -1,5 +1,5 @@
 """A stream module's stages in parts: generated from the spec as it is when it is
-generated."""
+generated, and for chains of stages of any length."""
 import copy
 
 from kunquant_gb300 import codegen
@@ -22,3 +22,15 @@ def test_a_spec_changed_in_place_is_generated_anew(tmp_path):
     ops.append(out)
     again = _sources(spec, tmp_path / "again")
     assert again == _sources(copy.deepcopy(spec), tmp_path / "copy") != short
+
+
+def test_a_long_chain_of_stages():
+    n = 3000
+    stages = [{"kind": "rank", "in": [k], "out": [k + 1]} for k in range(n)]
+    stages.append({"kind": "ts", "in": [n], "out": [n + 1],
+                   "ops": [{"k": "Input", "in": [], "buf": n}, {"k": "Abs", "in": [0]},
+                           {"k": "Output", "in": [1], "buf": n + 1}]})
+    # stages in any order: the last reads what the first ones lead to
+    for order in (stages, stages[::-1]):
+        si = order.index(stages[-1])
+        assert tick_groups({"stages": order}) == {si: [[[1, 2]]]}
