@@ -550,7 +550,9 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
         for (auto &hc : host_out) ptrs[hc.buf] = (char *)ex->staging.ptr + hc.off;
     }
     int64_t launches = 0;
-    // graph key: module, shape and every device address the kernels see
+    // graph key: module, shape, plan and every device address the kernels see
+    // (a run whose plan in kernels no longer fits goes on with the one in stages,
+    // in a smaller arena that may lie where the larger one did)
     std::vector<void *> gkey(ptrs.begin(), ptrs.end());
     gkey.push_back((void *)m);
     gkey.push_back((void *)(intptr_t)S);
@@ -559,6 +561,8 @@ KunStatus run_graph(Executor *ex, const KunGpuModuleDesc *m, const NameMap &name
     gkey.push_back((void *)(intptr_t)length);
     gkey.push_back(ex->arena.ptr);
     gkey.push_back((void *)(intptr_t)nstreams);
+    gkey.push_back((void *)(intptr_t)plan.num_slots);
+    gkey.push_back((void *)(intptr_t)plan.nodes.size());
     KunStatus rs = KUN_SUCCESS;
     GraphEntry *ge = nullptr;
     auto failed = [&](KunStatus status) {
