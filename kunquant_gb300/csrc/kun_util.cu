@@ -27,6 +27,12 @@
 namespace kungpu {
 
 constexpr int kCorrThreads = 256;
+// (row, input) pairs up to which an unranked call is one launch, in which every
+// input sums the label row again: launches cost more than that until the pairs
+// are some blocks an SM (us, one launch and three: 1 input of 5000 x 20 54 and 71,
+// 8 of 100 x 250 123 and 135, 8 of 5000 x 250 156 and 164, 32 of 5000 x 250 483
+// and 437).  Calls of one or two inputs are at any length (3000 x 1250 71 and 86).
+constexpr long long kCorrWhole = 2048;
 
 // element (t, s) of a [T][S] (layout 1) or [S/L][T][L] (layout 0) buffer
 __device__ __forceinline__ long long util_index(int layout, long long s, long long t, long long S, long long T,
@@ -95,21 +101,36 @@ __global__ void __launch_bounds__(kCorrThreads) corr_label_rows(const float *__r
 struct CorrRow {
     float x[2], x2[2], xy[2];
 };
-__device__ __forceinline__ void corr_add(CorrSums<3> &a, float x, float y) {
+template <int N> __device__ __forceinline__ void corr_add(CorrSums<N> &a, float x, float y) {
     a.v[0] = kun::df_add_f(a.v[0], x);
     a.v[1] = kun::df_add_prod(a.v[1], x, x);
     a.v[2] = kun::df_add_prod(a.v[2], x, y);
+    if constexpr (N == 5) {  // and the label row's own
+        a.v[3] = kun::df_add_f(a.v[3], y);
+        a.v[4] = kun::df_add_prod(a.v[4], y, y);
+    }
 }
-__device__ __forceinline__ void corr_store(const CorrSums<3> &a, CorrRow *o) {
-    *o = CorrRow{{a.v[0].hi, a.v[0].lo}, {a.v[1].hi, a.v[1].lo}, {a.v[2].hi, a.v[2].lo}};
+__device__ __forceinline__ CorrRow corr_row(const kun::DFloat *v) {
+    return CorrRow{{v[0].hi, v[0].lo}, {v[1].hi, v[1].lo}, {v[2].hi, v[2].lo}};
+}
+// (XY - X*Y) / (sqrt(X2 - X*X) * sqrt(Y2 - Y*Y)) of the means, in double from
+// the two-float sums (q: the label row's two)
+__device__ __forceinline__ float corr_of(const CorrRow &r, float4 q, long long S) {
+    const double n = (double)S;
+    const double mx = ((double)r.x[0] + r.x[1]) / n, my = ((double)q.x + q.y) / n;
+    const double mx2 = ((double)r.x2[0] + r.x2[1]) / n, my2 = ((double)q.z + q.w) / n;
+    const double mxy = ((double)r.xy[0] + r.xy[1]) / n;
+    return (float)((mxy - mx * my) / (sqrt(mx2 - mx * mx) * sqrt(my2 - my * my)));
 }
 
+// WHOLE: the label row's sums and the correlation too, in one launch
+template <bool WHOLE>
 __global__ void __launch_bounds__(kCorrThreads) corr_rows(const float *const *in, const float *__restrict__ y,
-                                                          CorrRow *__restrict__ sums, long long S, long long T,
-                                                          int layout, int L) {
+                                                          CorrRow *__restrict__ sums, float *const *out, long long S,
+                                                          long long T, int layout, int L) {
     const long long t = blockIdx.x;
     const float *__restrict__ x = in[blockIdx.y];
-    CorrSums<3> a;
+    CorrSums<WHOLE ? 5 : 3> a;
     if (layout == 1) {
         const float *__restrict__ xr = x + t * S, *__restrict__ yr = y + t * S;
 #pragma unroll 4
@@ -121,7 +142,11 @@ __global__ void __launch_bounds__(kCorrThreads) corr_rows(const float *const *in
         }
     }
     a.template reduce<true>(kCorrThreads);
-    if (threadIdx.x == 0) corr_store(a, sums + (long long)blockIdx.y * T + t);
+    if (threadIdx.x != 0) return;
+    if constexpr (WHOLE)
+        out[blockIdx.y][t] = corr_of(corr_row(a.v), make_float4(a.v[3].hi, a.v[3].lo, a.v[4].hi, a.v[4].lo), S);
+    else
+        sums[(long long)blockIdx.y * T + t] = corr_row(a.v);
 }
 
 // the same with every input row's ranks in place of its values: they are
@@ -158,23 +183,15 @@ __global__ void __launch_bounds__(MAXT, kun::rank_min_blocks<float>(16, MAXT))
     CorrSums<3> a;
     kun::rank_row<float, ITEMS>(in[blockIdx.y] + t * S, S, (int)blockDim.x, smem_raw, CorrRankAdd{a, y + t * S});
     a.template reduce<false>(blockDim.x);
-    if (threadIdx.x == 0) corr_store(a, sums + (long long)blockIdx.y * T + t);
+    if (threadIdx.x == 0) sums[(long long)blockIdx.y * T + t] = corr_row(a.v);
 }
 
-// (XY - X*Y) / (sqrt(X2 - X*X) * sqrt(Y2 - Y*Y)) of the means, in double from
-// the two-float sums.  One thread a (row, input): a block's one thread doing
-// it at the end of its row would hold the block for the double divisions.
+// One thread a (row, input): a block's one thread doing it at the end of its row
+// would hold the block for the double divisions.
 __global__ void corr_finish(const CorrRow *__restrict__ sums, const float4 *__restrict__ ysum, float *const *out,
                             long long S, long long T) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    const CorrRow r = sums[(long long)blockIdx.y * T + t];
-    const float4 q = ysum[t];
-    const double n = (double)S;
-    const double mx = ((double)r.x[0] + r.x[1]) / n, my = ((double)q.x + q.y) / n;
-    const double mx2 = ((double)r.x2[0] + r.x2[1]) / n, my2 = ((double)q.z + q.w) / n;
-    const double mxy = ((double)r.xy[0] + r.xy[1]) / n;
-    out[blockIdx.y][t] = (float)((mxy - mx * my) / (sqrt(mx2 - mx * mx) * sqrt(my2 - my * my)));
+    if (t < T) out[blockIdx.y][t] = corr_of(sums[(long long)blockIdx.y * T + t], ysum[t], S);
 }
 
 // First row of every run of equal consecutive labels (NaN equals nothing), in
@@ -340,7 +357,8 @@ KUN_EXPORT KunStatus kunCorrWith(KunExecutorHandle exec, int n, const float *con
     const long long S = (long long)num_stocks, T = (long long)num_time;
     cudaMemcpyAsync(d_in, inputs, (size_t)n * sizeof(void *), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d_out, outs, (size_t)n * sizeof(void *), cudaMemcpyHostToDevice, st);
-    corr_label_rows<<<(unsigned)T, kCorrThreads, 0, st>>>(corr_with, d_ysum, S, T, layout, 8);
+    const bool whole = !rank_inputs && (n <= 2 || n * T <= kCorrWhole);
+    if (!whole) corr_label_rows<<<(unsigned)T, kCorrThreads, 0, st>>>(corr_with, d_ysum, S, T, layout, 8);
     const dim3 grid((unsigned)T, (unsigned)n);
     if (rank_inputs) {
         const int rc = kun::rank_dispatch<false>(S, [&](auto items, auto maxt) {
@@ -355,10 +373,12 @@ KUN_EXPORT KunStatus kunCorrWith(KunExecutorHandle exec, int n, const float *con
             set_error("corrWith: rank failed: %s", cudaGetErrorString((cudaError_t)rc));
             return KUN_CUDA_ERROR;
         }
+    } else if (whole) {
+        corr_rows<true><<<grid, kCorrThreads, 0, st>>>(d_in, corr_with, nullptr, d_out, S, T, layout, 8);
     } else {
-        corr_rows<<<grid, kCorrThreads, 0, st>>>(d_in, corr_with, d_sums, S, T, layout, 8);
+        corr_rows<false><<<grid, kCorrThreads, 0, st>>>(d_in, corr_with, d_sums, nullptr, S, T, layout, 8);
     }
-    corr_finish<<<dim3((unsigned)((T + 127) / 128), (unsigned)n), 128, 0, st>>>(d_sums, d_ysum, d_out, S, T);
+    if (!whole) corr_finish<<<dim3((unsigned)((T + 127) / 128), (unsigned)n), 128, 0, st>>>(d_sums, d_ysum, d_out, S, T);
     if (cudaError_t e = cudaGetLastError()) {
         set_error("corrWith: %s", cudaGetErrorString(e));
         return KUN_CUDA_ERROR;
