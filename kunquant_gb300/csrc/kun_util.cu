@@ -224,29 +224,57 @@ __global__ void __launch_bounds__(kStartThreads) group_starts(const void *const 
     }
 }
 
-// One thread a stock takes the groups that begin in the block's kAggRows rows,
+// One thread a stock takes the groups that begin in the block's tile of rows,
 // each from its first row to its last (which may lie in later blocks' rows),
 // kAggAhead rows loaded ahead of the sums.  Groups do not depend on each
 // other: one thread a stock walking all rows (40 blocks at 5000 stocks) waited
 // for one load at a time, 1.1 ms an input of 2500 rows; now bound by memory, 6
-// inputs in about 0.1 ms with monthly groups.  32 rows a block give every SM
-// blocks from a few hundred rows and 128 stocks on.
-constexpr int kAggRows = 32;
+// inputs in about 0.1 ms with monthly groups.  32 rows a tile, or 8 where those
+// leave SMs without blocks: a thread's groups of one row wait for each other (60
+// rows of 5000 stocks 49 us in tiles of 32, 40 in tiles of 8).
+// OWN: of up to kAggThreads rows every block finds the groups itself, for the
+// launch of group_starts is a tenth of so short a call (60 rows of 5000 stocks in
+// groups of 21: 39 us with it, 34 without).
 constexpr int kAggAhead = 8;
-template <typename T>
-__global__ void __launch_bounds__(128) aggregate_groups(const void *const *in_, T *const *outs_,
-                                                        const long long *starts_, const long long *groups_,
-                                                        long long S, long long length) {
+constexpr int kAggThreads = 128;
+template <typename T, bool OWN>
+__global__ void __launch_bounds__(kAggThreads) aggregate_groups(const void *const *in_, const void *const *labels,
+                                                                T *const *outs_, const long long *starts_,
+                                                                const long long *groups_, long long S,
+                                                                long long length, int tile_rows) {
+    __shared__ long long own[OWN ? kAggThreads + 1 : 1];
+    __shared__ unsigned heads[kAggThreads / 32];
+    long long groups;
+    if (OWN) {
+        const T *__restrict__ lab = (const T *)labels[blockIdx.z];
+        const int r = threadIdx.x, lane = r & 31, w = r >> 5;
+        const bool head = r < length && (r == 0 || lab[r] != lab[r - 1]);
+        const unsigned m = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) heads[w] = m;
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int k = 0; k < kAggThreads / 32; k++) {
+            const int n = __popc(heads[k]);
+            before += k < w ? n : 0;
+            all += n;
+        }
+        if (head) own[before + __popc(m & ((1u << lane) - 1))] = r;
+        if (r == 0) own[all] = length;
+        groups = all;
+        __syncthreads();
+    } else {
+        groups = groups_[blockIdx.z];
+    }
     const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
     const T *__restrict__ in = (const T *)in_[blockIdx.z] + s;
     T *const *outs = outs_ + 7 * blockIdx.z;
-    const long long *__restrict__ starts = starts_ + blockIdx.z * (length + 1);
-    const long long groups = groups_[blockIdx.z];
+    const long long *starts = OWN ? own : starts_ + blockIdx.z * (length + 1);
     T *sum = outs[0], *mn = outs[1], *mx = outs[2], *first = outs[3], *last = outs[4], *cnt = outs[5],
       *mean = outs[6];
-    for (long long tile = blockIdx.y; tile * kAggRows < length; tile += gridDim.y) {
-        const long long r0 = tile * kAggRows, r1 = r0 + kAggRows < length ? r0 + kAggRows : length;
+    for (long long tile = blockIdx.y; tile * tile_rows < length; tile += gridDim.y) {
+        const long long r0 = tile * tile_rows, r1 = r0 + tile_rows < length ? r0 + tile_rows : length;
         long long g = 0, hi = groups;  // the first group that begins at r0 or later
         while (g < hi) {
             const long long m = (g + hi) >> 1;
@@ -426,13 +454,22 @@ KUN_EXPORT KunStatus kunAggregrate(KunExecutorHandle exec, int n, const void *co
     cudaMemcpyAsync(d_ptrs, table.data(), table.size() * sizeof(void *), cudaMemcpyHostToDevice, st);
     auto go = [&](auto zero) {
         using T = decltype(zero);
-        const long long S = (long long)num_stocks, rows = (long long)length, tiles = (rows + kAggRows - 1) / kAggRows;
-        group_starts<T><<<(unsigned)n, kStartThreads, 0, st>>>(d_ptrs + n, d_starts, d_groups, rows);
+        const long long S = (long long)num_stocks, rows = (long long)length;
+        const long long stock_blocks = (S + kAggThreads - 1) / kAggThreads;
+        const int tile_rows = stock_blocks * ((rows + 31) / 32) * n < 4LL * kun::kun_num_sms() ? 8 : 32;
+        const long long tiles = (rows + tile_rows - 1) / tile_rows;
+        const bool own = rows <= kAggThreads;
+        if (!own) group_starts<T><<<(unsigned)n, kStartThreads, 0, st>>>(d_ptrs + n, d_starts, d_groups, rows);
         for (int k = 0; k < n; k += 65535) {
-            const dim3 grid((unsigned)((S + 127) / 128), (unsigned)std::min(tiles, 65535LL),
+            const dim3 grid((unsigned)stock_blocks, (unsigned)std::min(tiles, 65535LL),
                             (unsigned)std::min(n - k, 65535));
-            aggregate_groups<T><<<grid, 128, 0, st>>>(d_ptrs + k, (T *const *)(d_ptrs + 2 * (size_t)n) + 7 * (size_t)k,
-                                                      d_starts + k * (rows + 1), d_groups + k, S, rows);
+            T *const *to = (T *const *)(d_ptrs + 2 * (size_t)n) + 7 * (size_t)k;
+            if (own)
+                aggregate_groups<T, true><<<grid, kAggThreads, 0, st>>>(d_ptrs + k, d_ptrs + n + k, to, nullptr, nullptr,
+                                                                        S, rows, tile_rows);
+            else
+                aggregate_groups<T, false><<<grid, kAggThreads, 0, st>>>(
+                    d_ptrs + k, nullptr, to, d_starts + k * (rows + 1), d_groups + k, S, rows, tile_rows);
         }
     };
     if (dtype == 0)
