@@ -182,9 +182,12 @@ struct StageBlocks {
     std::vector<std::vector<void *>> scratch;
     std::vector<KunGpuStageArgs> args;
     std::vector<size_t> off;  // per group of KUN_GROUP_MAX jobs
-    // the grouped Rank's launches: jobs of like length, so that a block has
-    // the threads and shared memory its rows need (12 universes of 37 to 3000
-    // stocks in one launch of 384-thread blocks: 104 us a stage, 57 in four)
+    // the grouped Rank's launches: jobs of like length, so that a block has the
+    // threads and shared memory its rows need.  A class more costs 2 to 5 us a
+    // stage, a wide one costs blocks that its short rows leave idle (us a stage,
+    // these four classes and one: 48 universes of 37 to 6000 stocks x 250 to 5000
+    // days 1613 and 2786; 12 of 37 to 3000 x 250 to 1250 149 and 152; 24 of 400 to
+    // 600 x 1000 230 and 228).
     struct RankClass {
         int first, jobs;
         long long rows, longest;
