@@ -51,10 +51,10 @@ template <int N> struct CorrSums {
     template <bool IN_ORDER> __device__ __forceinline__ void reduce(int nt) {
         __shared__ float sh[N][2][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = nt >> 5;
+        warp_totals();
+        if (lane == 0) {
 #pragma unroll
-        for (int q = 0; q < N; q++) {
-            butterfly(v[q]);
-            if (lane == 0) {
+            for (int q = 0; q < N; q++) {
                 sh[q][0][w] = v[q].hi;
                 sh[q][1][w] = v[q].lo;
             }
@@ -68,18 +68,38 @@ template <int N> struct CorrSums {
             for (int q = 0; q < N; q++) v[q] = across(total, q);
         } else {
 #pragma unroll
-            for (int q = 0; q < N; q++) {
-                v[q] = lane < nw ? kun::DFloat(sh[q][0][lane], sh[q][1][lane]) : kun::DFloat();
-                butterfly(v[q]);
-            }
+            for (int q = 0; q < N; q++) v[q] = lane < nw ? kun::DFloat(sh[q][0][lane], sh[q][1][lane]) : kun::DFloat();
+            warp_totals();
         }
     }
     static __device__ __forceinline__ kun::DFloat across(kun::DFloat x, int from) {
         return kun::DFloat(__shfl_sync(0xffffffffu, x.hi, from), __shfl_sync(0xffffffffu, x.lo, from));
     }
-    static __device__ __forceinline__ void butterfly(kun::DFloat &x) {
+    static __device__ __forceinline__ kun::DFloat pick(bool c, kun::DFloat x, kun::DFloat y) {
+        return kun::DFloat(c ? x.hi : y.hi, c ? x.lo : y.lo);
+    }
+    // the warp's sums in every lane.  Of three, each lane goes on with the one
+    // that its half and quarter keep: the butterfly's additions (which give the
+    // same in either order) in 6 instead of 15.
+    __device__ __forceinline__ void warp_totals() {
+        const int lane = threadIdx.x & 31;
+        if constexpr (N == 3) {
+            const bool low = lane < 16, first = (lane & 8) == 0;
+            const kun::DFloat a = across(pick(low, v[2], v[0]), lane ^ 16), b = across(v[1], lane ^ 16);
+            const kun::DFloat x = kun::kadd(pick(low, v[0], v[2]), a), y = kun::kadd(v[1], b);
+            const kun::DFloat send = pick(low && first, y, x), keep = pick(low && !first, y, x);
+            kun::DFloat t = kun::kadd(keep, across(send, lane ^ 8));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = kun::kadd(x, across(x, (threadIdx.x & 31) ^ o));
+            for (int o = 4; o > 0; o >>= 1) t = kun::kadd(t, across(t, lane ^ o));
+            v[0] = across(t, 0);
+            v[1] = across(t, 8);
+            v[2] = across(t, 16);
+        } else {
+#pragma unroll
+            for (int q = 0; q < N; q++)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v[q] = kun::kadd(v[q], across(v[q], lane ^ o));
+        }
     }
 };
 
@@ -152,7 +172,7 @@ __global__ void __launch_bounds__(kCorrThreads) corr_rows(const float *const *in
 // the same with every input row's ranks in place of its values: they are
 // summed where kun::rank_row finds them and never reach memory (5000 stocks x
 // 1250 days x 32 inputs wrote and read 1.6 GB of them, in 33 launches: 5.4 ms,
-// now 2.4 ms, bound by the ranking).  Ranks lie in (0, 1] and a thread has at
+// now 2.2 ms, bound by the ranking).  Ranks lie in (0, 1] and a thread has at
 // most 16, so an addition takes the low parts together before it normalises:
 // half the instructions, and with the butterfly over the warps an error no
 // larger than that of the full additions of 256 threads (restated on the CPU, 100
