@@ -300,19 +300,22 @@ KunStatus enqueue_tick(const StreamStore &store, const std::vector<int> &order, 
                        const TickLevels *levels) {
     const KunGpuModuleDesc *m = store.m;
     if (levels && levels->ok) {
-        // Rank over a device table's segments: a launch for the short ones beside
-        // one for the long ones, of which the step's stocks allow a few only.  A
-        // block with the threads and shared memory of the longest segment fills
-        // an SM whatever it ranks (256 sessions of 64 stocks in a pool that takes
-        // 16384: 1140 us a step in one launch, 594 in two).
-        // (A pool for longer rows than Rank takes is refused whatever its step.)
+        // Rank over a device table's segments: where they are many, a launch for
+        // the short ones beside one for the long ones, of which the step's stocks
+        // allow a few only.  A block with the threads and shared memory of the
+        // longest segment fills an SM whatever it ranks (256 sessions of 64 stocks
+        // in a pool that takes 16384: 1140 us a step in one launch, 594 in two);
+        // few blocks are there together anyway, and one launch a level is the
+        // shorter chain (16 sessions of 100 to 5000: 420 us, 428 in two).  (A pool
+        // for longer rows than Rank takes is refused whatever its step.)
         const int longest = max_len > kun::kRankMaxStocks ? max_len : (int)std::min<long long>(max_len, n_active);
         const bool both = d_seg_count && longest > kun::kRankShort;
         const auto &side = levels->ex->side;
         for (size_t l = 0; l < levels->other.size(); l++) {
             // the level's first launch stays on the tick's stream
             const auto &units = levels->other[l];
-            const bool ranks = levels->rank_cnt[l] > 0, two = ranks && both;
+            const bool ranks = levels->rank_cnt[l] > 0;
+            const bool two = ranks && both && (long long)nseg * levels->rank_cnt[l] > 4LL * kun::kun_num_sms();
             const size_t here = ranks ? 0 : 1;
             const size_t beside = (units.size() > here ? units.size() - here : 0) + two;
             const size_t sides = std::min(beside, side.size());
