@@ -67,9 +67,11 @@ typedef struct {
  * on the current CUDA device with one stream. */
 KunExecutorHandle kunCreateSingleThreadExecutor(void);
 /* Replaces kunCreateMultiThreadExecutor (cpp/Kun/CApi.h:57): `numthreads` is
- * the number of CUDA streams used to run independent stages concurrently. */
+ * the number of CUDA streams used to run independent stages concurrently; runs
+ * of an executor of two or more use 24 streams if it is fewer. */
 KunExecutorHandle kunCreateMultiThreadExecutor(int numthreads);
-/* cpp/Kun/CApi.h:65 (sic: "Destory" as in the reference) */
+/* cpp/Kun/CApi.h:65 (sic: "Destory" as in the reference).  The streams and
+ * serving pools made on it keep it until they are destroyed. */
 void kunDestoryExecutor(KunExecutorHandle ptr);
 
 /* cpp/Kun/CApi.h:73: load a GPU module library (.so) */
