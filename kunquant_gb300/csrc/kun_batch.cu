@@ -436,7 +436,7 @@ KUN_EXPORT KunStatus kunRunGraphBatch(KunExecutorHandle exec, KunModuleHandle mo
 // {default, 16, 32, 64, 128, 256} x {64, 128} threads per block for all the
 // time-parallel kernels of a stage together, {32, 64, 128} threads for its
 // scan kernels; then per time-parallel kernel, with the others held: its
-// 64-register instance or not x block size, then its tile.  Each candidate
+// 64-register instance (if it has one) or not x block size, then its tile.  Each candidate
 // runs the stage `reps` times after one warm-up; the fastest mean wins.
 // Returns the number of stages tuned, or -1 on error.
 KUN_EXPORT int kunExecutorTune(KunExecutorHandle exec, KunModuleHandle mod, int njobs,
@@ -540,6 +540,7 @@ KUN_EXPORT int kunExecutorTune(KunExecutorHandle exec, KunModuleHandle mod, int 
         for (int k = 0; k < nk && has_par; k++) {
             if (d.kernel_info[k] & 1) continue;
             for (int cap : {0, (int)KUN_BLOCK_REGCAP}) {
+                if (cap && !(d.kernel_info[k] & KUN_KERNEL_CAPPED)) continue;
                 for (int blk : blocks) {
                     t = best_t;
                     b = best_b;

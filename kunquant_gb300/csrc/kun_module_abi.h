@@ -13,6 +13,7 @@ extern "C" {
 
 #define KUN_GPU_MODULE_ABI 0x6b47000aull
 #define KUN_BLOCK_REGCAP 0x10000
+#define KUN_KERNEL_CAPPED 0x40000000
 
 typedef enum { KUN_LAYOUT_STS = 0, KUN_LAYOUT_TS = 1, KUN_LAYOUT_STREAM = 2 } KunGpuLayout;
 typedef enum { KUN_BUF_INPUT = 0, KUN_BUF_OUTPUT = 1, KUN_BUF_TEMP = 2 } KunGpuBufferKind;
@@ -105,7 +106,8 @@ typedef struct {
      * kernel reads them.  NULL when state_i_vars is 0. */
     const int32_t *state_i_max;
     /* time-series stages with grouped launches: per kernel, default time
-     * tile << 1 (or number of scan roles << 1) | 1 for a scan kernel.  Behind
+     * tile << 1 (or number of scan roles << 1) | 1 for a scan kernel |
+     * KUN_KERNEL_CAPPED for one that has a 64-register instance.  Behind
      * these num_kernels entries, per kernel: the instructions a cell takes
      * (an estimate), the number of series it reads from other kernels and
      * those, the number it writes and those; a series is a buffer id, or

@@ -473,6 +473,8 @@ VEC_U = 4
 # rows a thread computes at once in a kernel without window loops, where
 # the rows share no loads and more of them only cost registers
 VEC_U_ELEM = 2
+# in the module table: the kernel has a 64-register instance (KUN_KERNEL_CAPPED)
+KERNEL_CAPPED = 1 << 30
 # rows a window queue loads ahead of use, and the unroll of the loops over
 # windows (10 divides the usual windows: 5 to 20% on a kernel of window sums
 # against 4) and over the common run of window extremes (their branches grow
@@ -1795,7 +1797,7 @@ struct {pstruct} {{
   int* err;
 }};
 """
-        self.kernel_info = [(d << 1) | sc for d, sc in kinfo]
+        self.kernel_info = [(d << 1) | sc | (KERNEL_CAPPED if k in capped else 0) for k, (d, sc) in enumerate(kinfo)]
         for kd in ks:
             self.kernel_info += self._kernel_io(kd)
         self.num_kernels_override = nk

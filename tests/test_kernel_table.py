@@ -97,6 +97,22 @@ def test_table_has_what_the_kernels_touch(key, tmp_path):
     assert checked > 50, checked
 
 
+@pytest.mark.parametrize("key", ["alpha158_f32", "alpha158_slide_f32", "alpha101_f32"])
+def test_table_says_which_kernels_have_a_capped_instance(key, tmp_path):
+    spec = predefined_spec(key)
+    tag = spec["name"]
+    src = "\n".join(open(p).read() for p in codegen.generate_module(spec, str(tmp_path), tag=tag))
+    seen = set()
+    for m in re.finditer(r"st(\d+)_kinfo\[\] = \{([^}]*)\}", src):
+        prefix = f"kst_{tag}_{m.group(1)}"
+        info = [int(v) for v in m.group(2).split(",")]
+        for k in _functions(src, prefix):
+            capped = re.search(r"%s_L\d+_%d_r\(" % (re.escape(prefix), k), src) is not None
+            assert bool(info[k] & 0x40000000) == capped, (prefix, k)
+            seen.add(capped)
+    assert seen == {False, True}
+
+
 def test_the_check_sees_a_missing_read(tmp_path):
     text = "  const float* __restrict__ b3 = (const float*)P.p[2] + s;\n  float* __restrict__ b4 = (float*)P.w[7] + s;\n" \
            "  b4[(t + u) * st4] = kun::ldw<KE>(b3, st3, (long long)(t + u), length) + b4[(t - 1) * st4];"
